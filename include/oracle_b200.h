@@ -127,7 +127,17 @@ extern "C" {
                              * (their divergence is linear in the stage's sdt), each
                              * stage's y pencils forming its spectrum; z-chunk, 0 = off;
                              * takes effect with the 1024-point y pencils (zc4_fy) */
-#define OB_VAR_COUNT 23
+/* The level-paired line transforms (any nx, ny whose halves have no factor
+ * above 5), 0 or 1 per class; a class whose entry is 1 runs them whatever its
+ * other entries are.  _FXD / _FYD: the FP64 residual transforms. */
+#define OB_VAR_Z_FX 23
+#define OB_VAR_Z_FXS 24
+#define OB_VAR_Z_IX 25
+#define OB_VAR_Z_FY 26
+#define OB_VAR_Z_IY 27
+#define OB_VAR_Z_FXD 28
+#define OB_VAR_Z_FYD 29
+#define OB_VAR_COUNT 30
 
 #define OB_TUNE_FORCE 1  /* time the candidates even when a choice is cached */
 
@@ -481,8 +491,9 @@ const char *oracle_b200_last_error(void);
  * whenever a constant, an array length or a struct of this header changes, so
  * that bindings can refuse a library built from another header.  2: the
  * shared stage transforms (OB_VAR_ZC4_FXSH, OB_VAR_COUNT 23) and the
- * long-wave Thomas profile class (OB_PROF_THOMAS_LW, OB_PROF_CLASSES 10). */
-#define OB_ABI_VERSION 2
+ * long-wave Thomas profile class (OB_PROF_THOMAS_LW, OB_PROF_CLASSES 10).  3:
+ * the level-paired line transforms (OB_VAR_Z_*, OB_VAR_COUNT 30). */
+#define OB_ABI_VERSION 3
 int oracle_b200_version(void);
 
 #ifdef __cplusplus

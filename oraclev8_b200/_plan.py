@@ -215,9 +215,9 @@ class Plan:
         L.check(self.lib.oracle_b200_plan_set_variants(self.handle, vals, len(L.VARIANTS)))
 
     def shared_memory_forms(self) -> None:
-        """Turn every register-resident and compile-time-chunk form off: the
-        runtime-chunk shared-memory Stockham kernels only."""
-        self.set_variants(**{k: 0 for k in L.VARIANTS if k.startswith(("zc3", "zc4"))})
+        """Turn every register-resident and level-paired form off: the
+        shared-memory Stockham kernels only."""
+        self.set_variants(**{k: 0 for k in L.VARIANTS if k.startswith(("zc3", "zc4", "z_"))})
 
     def tune(self, force: bool = False) -> dict:
         """Time the kernel forms of each class and keep the fastest (cached per

@@ -11,18 +11,23 @@ import os
 import shutil
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 ROOT = PKG.parent
 CSRC = PKG / "csrc"
 LIB = PKG / "liboracle_b200.so"
-SOURCES = [CSRC / "api.cu"]
-DEPS = SOURCES + sorted(CSRC.glob("*.cuh")) + [ROOT / "include" / "oracle_b200.h"]
+# translation units: (source, defines), compiled side by side
+UNITS = [(CSRC / "api.cu", ())] + [
+    (CSRC / "zfft.cu", (f"-DOB_ZREAL={real}", f"-DOB_ZELEM={elem}", f"-DOB_ZPART={part}"))
+    for real, elem in (("float", 4), ("double", 8)) for part in (0, 2, 4, 6, 8)]
+DEPS = (sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h"))
+        + [ROOT / "include" / "oracle_b200.h"])
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
-         "-shared", "-Xptxas", "-warn-spills"]
+FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xptxas", "-warn-spills"]
 
 
 def nvcc() -> str:
@@ -43,11 +48,20 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if not force and up_to_date():
         return LIB
     tmp = LIB.with_suffix(".so.tmp")
-    cmd = [nvcc(), *ARCH, *FLAGS, "-o", str(tmp), *map(str, SOURCES), "-lcudart"]
-    if verbose:
-        cmd.insert(1, "-Xptxas=-v")
-        print(" ".join(cmd), flush=True)
-    subprocess.run(cmd, check=True)
+    flags = FLAGS + (["-Xptxas=-v"] if verbose else [])
+    with tempfile.TemporaryDirectory() as d:
+        def unit(i):
+            src, defines = UNITS[i]
+            obj = Path(d) / f"{src.stem}_{i}.o"
+            cmd = [nvcc(), *ARCH, *flags, *defines, "-c", "-o", str(obj), str(src)]
+            if verbose:
+                print(" ".join(cmd), flush=True)
+            subprocess.run(cmd, check=True)
+            return str(obj)
+
+        with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+            objs = list(pool.map(unit, range(len(UNITS))))
+        subprocess.run([nvcc(), *ARCH, "-shared", "-o", str(tmp), *objs, "-lcudart"], check=True)
     os.replace(tmp, LIB)
     return LIB
 

@@ -21,6 +21,7 @@
 #include "tracker.cuh"
 #include "vdiag.cuh"
 #include "init.cuh"
+#include "zfft.h"
 
 using namespace ob;
 
@@ -232,6 +233,13 @@ struct OraclePlan {
   // (k_fx4 with four column groups into S4..S6, then k_fy4 forming each
   // stage's divergence spectrum): its z-chunk, 0 = off; needs zc4_fy
   int zc4_fxsh = 0;
+  // level-paired line transforms (zfft.cuh): line plans, tables in the plan's
+  // type (wavenumbers with the Nyquist entry zeroed), and per class whether the
+  // form is on; z_fxd / z_fyd: the FP64 residual transforms (the refiner's plan)
+  ZPlan zpx{}, zpy{};
+  bool zx_ok = false, zy_ok = false;
+  void *zkx = nullptr, *zky = nullptr, *ztx = nullptr, *zty = nullptr;
+  int z_fx = 0, z_fxs = 0, z_ix = 0, z_fy = 0, z_iy = 0, z_fxd = 0, z_fyd = 0;
   // FP32 slow tendency: 0 the gather form, 1 marching along x (k_slow_xw),
   // 4 / 8 marching along x over bulk-copied planes of 4 / 8 rows (k_slow_xt)
   int slow_xw = 1;
@@ -539,6 +547,7 @@ int set_smem_attrs() {
   OB_CUDA(cudaFuncSetAttribute(k_fx<double, FX_DIV, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
   OB_CUDA(cudaFuncSetAttribute(k_fy<double, FY_RESID, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
   OB_CUDA(cudaFuncSetAttribute(k_ix<float, IX_REFINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+  OB_CUDA(zfft_init<T>());
   return set_x2_attrs<T>();
 }
 
@@ -998,6 +1007,47 @@ void yr4(const OraclePlan* p, bool inverse, const cplx<float>* in0, const cplx<f
   }
 }
 
+// The plan's lines in x and y for the level-paired transforms.
+template <class T>
+ZLine<T> zline_x(const OraclePlan* p) {
+  return {p->zpx, (const T*)p->zkx, (const cplx<T>*)p->ztx};
+}
+template <class T>
+ZLine<T> zline_y(const OraclePlan* p) {
+  return {p->zpy, (const T*)p->zky, (const cplx<T>*)p->zty};
+}
+
+// Line plans and wavenumber tables of a plan (allocated from `owner`).
+template <class T>
+int make_zlines(OraclePlan* owner, OraclePlan* p, const double* kx, const double* ky) {
+  p->zx_ok = zplan_make(p->g.nx, (int)sizeof(T), &p->zpx);
+  p->zy_ok = zplan_make(p->g.ny, (int)sizeof(T), &p->zpy);
+  auto table = [&](void** out, const double* k, int n) {
+    std::vector<T> t(n);
+    for (int i = 0; i < n; ++i) t[i] = 2 * i == n ? (T)0 : (T)k[i];
+    if (int rc = dalloc(owner, out, n * sizeof(T))) return rc;
+    OB_CUDA(cudaMemcpyAsync(*out, t.data(), n * sizeof(T), cudaMemcpyHostToDevice,
+                            owner->astream));
+    return (int)OB_OK;
+  };
+  auto twid = [&](void** out, bool ok, const ZPlan& l) {
+    if (!ok) return (int)OB_OK;
+    std::vector<int> at(l.N);
+    zplan_twiddles(l, at.data());
+    const std::vector<cplx<T>> w = twiddles<T>(l.N);
+    std::vector<cplx<T>> t(l.N);
+    for (int i = 0; i < l.N; ++i) t[i] = w[at[i]];
+    if (int rc = dalloc(owner, out, l.N * sizeof(cplx<T>))) return rc;
+    OB_CUDA(cudaMemcpyAsync(*out, t.data(), l.N * sizeof(cplx<T>), cudaMemcpyHostToDevice,
+                            owner->astream));
+    return (int)OB_OK;
+  };
+  RC(table(&p->zkx, kx, p->g.nx));
+  RC(table(&p->zky, ky, p->g.ny));
+  RC(twid(&p->ztx, p->zx_ok, p->zpx));
+  return twid(&p->zty, p->zy_ok, p->zpy);
+}
+
 // The single-precision short-wave launch with a compile-time level count
 // (k_thomas_f32); false when nz has no instance.
 bool thomas_f32(OraclePlan* p, int cls, cplx<float>* S3, cudaStream_t st) {
@@ -1084,6 +1134,11 @@ int proj_fx(OraclePlan* p, bool stage, const T* u, const T* v, const T* w, const
   C* S1 = (C*)p->S1;
   C* S2 = (C*)p->S2;
   Launch L_(p, 0, st);
+  if (stage ? (bh && p->z_fxs) : p->z_fx) {
+    OB_CUDA((zfx<T, T>(stage ? ZFX_STAGE : ZFX_DIV, zline_x<T>(p), g, u, v, w, bh, sdt, p->rho,
+                       p->rhoh, S1, S2, nullptr, st)));
+    return OB_OK;
+  }
   if constexpr (sizeof(T) == 4) {
     if (stage && bh && p->zc4_fxs) {
       fx4<float, true>(p, p->zc4_fxs, u, v, w, bh, sdt, S1, S2, st);
@@ -1131,6 +1186,11 @@ int proj_fy(OraclePlan* p, cudaStream_t st) {
   C* S2 = (C*)p->S2;
   C* S3 = (C*)p->S3;
   Launch L_(p, 1, st);
+  if (p->z_fy) {
+    OB_CUDA((zfy<T, T>(ZFY_DIV, zline_y<T>(p), g, S1, S2, nullptr, 0.0, p->kx, p->ky, S3,
+                       nullptr, st)));
+    return OB_OK;
+  }
   if (sizeof(T) == 4 && p->zc4_fy)
     yr4(p, false, (const cplx<float>*)S1, (const cplx<float>*)S2, (cplx<float>*)S3, nullptr, st);
   else if (sizeof(T) == 4 && p->zc3_fy)
@@ -1153,6 +1213,10 @@ int proj_iy(OraclePlan* p, int cls, cudaStream_t st) {
   C* S2 = (C*)p->S2;
   C* S3 = (C*)p->S3;
   Launch L_(p, cls, st);
+  if (p->z_iy) {
+    OB_CUDA(ziy<T>(true, zline_y<T>(p), g, S3, 1.0, S1, S2, st));
+    return OB_OK;
+  }
   if (sizeof(T) == 4 && p->zc4_iy)
     yr4(p, true, (const cplx<float>*)S3, nullptr, (cplx<float>*)S1, (cplx<float>*)S2, st);
   else if (sizeof(T) == 4 && p->zc3_fy)
@@ -1175,6 +1239,11 @@ int proj_ix(OraclePlan* p, bool stage, const T* u, const T* v, const T* w, const
   C* S1 = (C*)p->S1;
   C* S2 = (C*)p->S2;
   Launch L_(p, 4, st);
+  if (p->z_ix && (bh || !stage)) {
+    OB_CUDA(zix<T>(stage ? ZIX_STAGE : ZIX_CORRECT, zline_x<T>(p), g, S1, S2, u, v, w, bh, sdt,
+                   uo, vo, wo, phio, st));
+    return OB_OK;
+  }
   if constexpr (sizeof(T) == 4) {
     if (p->zc4_ix && (bh || !stage)) {
       if (stage) ix4<IX_STAGE>(p, p->zc4_ix, S1, S2, u, v, w, bh, sdt, uo, vo, wo, phio, st);
@@ -1219,7 +1288,7 @@ int project_impl(OraclePlan* p, const T* u, const T* v, const T* w, const T* th,
   // a stage projection reads the half-level buoyancy in every form but the
   // generic one; without it a selected form would silently fall back
   if (stage_sdt >= 0.0 && !bh && (p->zc2_fxs || p->zc2_ix || p->zc3_fxs || p->zc3_ix || p->zc4_fxs ||
-                    p->zc4_ix))
+                    p->zc4_ix || p->z_fxs || p->z_ix))
     return fail(OB_ERR_CUDA, "stage projection without the half-level buoyancy its "
                 "kernel forms read");
   p->solve_count += 1;
@@ -1263,6 +1332,11 @@ int refine_fx(OraclePlan* p, const float* u, const float* v, const float* w, cud
   Cd* R1 = (Cd*)q->S1;
   Cd* R2 = (Cd*)q->S2;
   Launch L_(p, OB_PROF_REFINE, st);
+  if (p->z_fxd) {
+    OB_CUDA((zfx<double, float>(ZFX_DIV, zline_x<double>(q), g, u, v, w, nullptr, 0.0, p->rho,
+                                p->rhoh, R1, R2, nullptr, st)));
+    return OB_OK;
+  }
   if (p->zc4_fxd)
     fx4<double, false>(q, p->zc4_fxd, u, v, w, nullptr, 0.0, R1, R2, st);
   else if (p->zc3_fxd)
@@ -1286,6 +1360,11 @@ int refine_fy(OraclePlan* p, cudaStream_t st) {
   Cd* R2 = (Cd*)q->S2;
   cplx<float>* S3 = (cplx<float>*)p->S3;
   Launch L_(p, OB_PROF_REFINE, st);
+  if (p->z_fyd) {
+    OB_CUDA((zfy<double, float>(ZFY_RESID, zline_y<double>(q), g, R1, R2, nullptr, 0.0, q->kx,
+                                q->ky, S3, nullptr, st)));
+    return OB_OK;
+  }
   if (p->zc4_fyd) {
     const int items = ((g.nz + 1) / 2) * g.nxh;
     const int grid = std::min(items, resident_ctas(k_fy4d, 128, Yr4dSize::total));
@@ -1315,6 +1394,12 @@ int refine_impl(OraclePlan* p, float* u, float* v, float* w, float* phi, cudaStr
   RC(refine_fy(p, st));
   RC(thomas_solve<float>(p, OB_PROF_REFINE, S3, nullptr, 0, 0, st));
   RC(proj_iy<float>(p, OB_PROF_REFINE, st));
+  if (p->z_ix) {
+    Launch L_(p, OB_PROF_REFINE, st);
+    OB_CUDA(zix<float>(ZIX_REFINE, zline_x<float>(p), g, S1, S2, u, v, w, nullptr, 0.0, u, v, w,
+                       phi, st));
+    return OB_OK;
+  }
   if (p->zc4_ix)
     { Launch L_(p, OB_PROF_REFINE, st); ix4<IX_REFINE>(p, p->zc4_ix, S1, S2, u, v, w, nullptr, 0.0, u, v, w, phi, st); }
   else if (p->zc3_ix)
@@ -1332,7 +1417,7 @@ int refine_impl(OraclePlan* p, float* u, float* v, float* w, float* phi, cudaStr
 // Double-precision companion of a single-precision plan for the residual
 // transforms: FP64 twiddles and two FP64 half-spectrum buffers; the FFT
 // plans, wavenumbers and reference profiles are shared with the plan.
-int make_refiner(OraclePlan* p) {
+int make_refiner(OraclePlan* p, const double* kx, const double* ky) {
   OraclePlan* q = new OraclePlan();
   p->dbl = q;
   q->prec = OB_PREC_F64;
@@ -1368,6 +1453,9 @@ int make_refiner(OraclePlan* p) {
                           p->astream));
   const size_t ns = (size_t)p->g.nxh * ny * nz;
   if ((rc = dalloc(p, &q->S1, ns * ce)) || (rc = dalloc(p, &q->S2, ns * ce))) return rc;
+  RC(make_zlines<double>(p, q, kx, ky));
+  p->z_fxd = q->zx_ok;
+  p->z_fyd = q->zy_ok;
   return set_smem_attrs_once<double>();
 }
 
@@ -1378,7 +1466,10 @@ int damper_impl(OraclePlan* p, const T* u, const T* v, double dt_slow, cudaStrea
   const GridK g = p->g;
   C* S1 = (C*)p->S1;
   C* S2 = (C*)p->S2;
-  if (sizeof(T) == 4 && p->zc3_fx)
+  if (p->z_fx)
+    { Launch L_(p, 0, st); OB_CUDA((zfx<T, T>(ZFX_FIELDS, zline_x<T>(p), g, u, v, nullptr, nullptr,
+                                              0.0, p->rho, p->rhoh, S1, S2, nullptr, st))); }
+  else if (sizeof(T) == 4 && p->zc3_fx)
     { Launch L_(p, 0, st); fx3f(p, p->zc3_fx, (const float*)u, (const float*)v, (cplx<float>*)S1,
                                (cplx<float>*)S2, st); }
   else
@@ -1387,7 +1478,11 @@ int damper_impl(OraclePlan* p, const T* u, const T* v, double dt_slow, cudaStrea
         (const C*)p->twx, S1, S2, nullptr); }
   OB_LAUNCHED();
   const double scale = -(p->epsilon / dt_slow) / ((double)g.nx * (double)g.ny);
-  if (sizeof(T) == 4 && p->zc3_fy) {
+  if (p->z_fy) {
+    Launch L_(p, 1, st);
+    OB_CUDA((zfy<T, T>(ZFY_HELM, zline_y<T>(p), g, S1, S2, nullptr, scale, p->kx, p->ky, S1, S2,
+                       st)));
+  } else if (sizeof(T) == 4 && p->zc3_fy) {
     // forward y, multipliers and inverse y in one register-resident pass
     { Launch L_(p, 1, st); hy(p, scale, (cplx<float>*)S1, (cplx<float>*)S2, st); }
     OB_LAUNCHED();
@@ -1399,7 +1494,11 @@ int damper_impl(OraclePlan* p, const T* u, const T* v, double dt_slow, cudaStrea
       g, p->py, p->zc_iy, 2, S1, S2, p->ky, (const C*)p->twy, 1.0, S1, S2); }
   OB_LAUNCHED();
   }
-  if (sizeof(T) == 4 && p->zc3_ix)
+  if (p->z_ix)
+    { Launch L_(p, 4, st); OB_CUDA(zix<T>(ZIX_FIELDS, zline_x<T>(p), g, S1, S2, nullptr, nullptr,
+                                          nullptr, nullptr, 0.0, (T*)p->Du, (T*)p->Dv, nullptr,
+                                          nullptr, st)); }
+  else if (sizeof(T) == 4 && p->zc3_ix)
     { Launch L_(p, 4, st); ix3<IX_FIELDS>(p, p->zc3_ix, (const cplx<float>*)S1,
                                           (const cplx<float>*)S2, nullptr, nullptr, nullptr,
                                           nullptr, 0.0, (float*)p->Du, (float*)p->Dv, nullptr,
@@ -1740,29 +1839,56 @@ int step_impl(OraclePlan* p, const OracleStatePtrs* in, const OracleStatePtrs* o
   return OB_OK;
 }
 
+// One field's plain transforms (operator entry points): x forward into S1 and
+// S2 or S1 alone, y forward S1 -> S3, y inverse S3 -> S1, x inverse S1 -> out.
 template <class T>
-int divergence_impl(OraclePlan* p, const T* u, const T* v, const T* w, T* d, cudaStream_t st) {
+int op_fx_div(OraclePlan* p, const T* u, const T* v, const T* w, cudaStream_t st) {
   using C = cplx<T>;
-  const GridK g = p->g;
-  C* S1 = (C*)p->S1;
-  C* S2 = (C*)p->S2;
-  C* S3 = (C*)p->S3;
-  { Launch L_(p, 0, st); k_fx<T, FX_DIV><<<grid_x(p, p->zc_fx), kFftThreads, smem_fx(p, 3), st>>>(
-      g, p->pxf, p->zc_fx, 3, u, v, w, nullptr, 0.0, p->rho, p->rhoh, p->theta0, p->kx,
-      (const C*)p->twx, S1, S2, nullptr); }
-  OB_LAUNCHED();
-  { Launch L_(p, 1, st); k_fy<T, FY_DIV><<<grid_y(p, p->zc_fy), kFftThreads, smem_fy(p, 2, p->zc_fy), st>>>(
-      g, p->pyf, p->zc_fy, 2, S1, S2, p->kx, p->ky, (const C*)p->twy, 1.0, S3, nullptr); }
-  OB_LAUNCHED();
-  { Launch L_(p, 3, st); k_iy<T, IY_FIELDS><<<grid_y(p, p->zc_iy), kFftThreads, smem_fy(p, 2, p->zc_iy), st>>>(
-      g, p->py, p->zc_iy, 1, S3, nullptr, p->ky, (const C*)p->twy,
-      1.0 / ((double)g.nx * (double)g.ny), S1, nullptr); }
-  OB_LAUNCHED();
-  { Launch L_(p, 4, st); k_ix<T, IX_FIELDS><<<grid_x(p, p->zc_ix), kFftThreads, smem_ix(p, 2 * p->zc_ix), st>>>(
-      g, p->px, p->zc_ix, 1, S1, nullptr, nullptr, p->kx, (const C*)p->twx, nullptr, nullptr,
-      nullptr, nullptr, 0.0, p->theta0, d, nullptr, nullptr, nullptr); }
+  Launch L_(p, 0, st);
+  if (p->z_fx)
+    OB_CUDA((zfx<T, T>(ZFX_DIV, zline_x<T>(p), p->g, u, v, w, nullptr, 0.0, p->rho, p->rhoh,
+                       (C*)p->S1, (C*)p->S2, nullptr, st)));
+  else
+    k_fx<T, FX_DIV><<<grid_x(p, p->zc_fx), kFftThreads, smem_fx(p, 3), st>>>(
+        p->g, p->pxf, p->zc_fx, 3, u, v, w, nullptr, 0.0, p->rho, p->rhoh, p->theta0, p->kx,
+        (const C*)p->twx, (C*)p->S1, (C*)p->S2, nullptr);
   OB_LAUNCHED();
   return OB_OK;
+}
+template <class T>
+int op_iy_field(OraclePlan* p, double scale, cudaStream_t st) {
+  using C = cplx<T>;
+  Launch L_(p, 3, st);
+  if (p->z_iy)
+    OB_CUDA(ziy<T>(false, zline_y<T>(p), p->g, (C*)p->S3, scale, (C*)p->S1, nullptr, st));
+  else
+    k_iy<T, IY_FIELDS><<<grid_y(p, p->zc_iy), kFftThreads, smem_fy(p, 2, p->zc_iy), st>>>(
+        p->g, p->py, p->zc_iy, 1, (C*)p->S3, nullptr, p->ky, (const C*)p->twy, scale, (C*)p->S1,
+        nullptr);
+  OB_LAUNCHED();
+  return OB_OK;
+}
+template <class T>
+int op_ix_field(OraclePlan* p, T* out, cudaStream_t st) {
+  using C = cplx<T>;
+  Launch L_(p, 4, st);
+  if (p->z_ix)
+    OB_CUDA(zix<T>(ZIX_FIELDS, zline_x<T>(p), p->g, (C*)p->S1, nullptr, nullptr, nullptr, nullptr,
+                   nullptr, 0.0, out, nullptr, nullptr, nullptr, st));
+  else
+    k_ix<T, IX_FIELDS><<<grid_x(p, p->zc_ix), kFftThreads, smem_ix(p, 2 * p->zc_ix), st>>>(
+        p->g, p->px, p->zc_ix, 1, (C*)p->S1, nullptr, nullptr, p->kx, (const C*)p->twx, nullptr,
+        nullptr, nullptr, nullptr, 0.0, p->theta0, out, nullptr, nullptr, nullptr);
+  OB_LAUNCHED();
+  return OB_OK;
+}
+
+template <class T>
+int divergence_impl(OraclePlan* p, const T* u, const T* v, const T* w, T* d, cudaStream_t st) {
+  RC(op_fx_div<T>(p, u, v, w, st));
+  RC(proj_fy<T>(p, st));
+  RC(op_iy_field<T>(p, 1.0 / ((double)p->g.nx * (double)p->g.ny), st));
+  return op_ix_field<T>(p, d, st);
 }
 
 // forward 2-D real FFT of one field into S3 (unnormalised)
@@ -1770,45 +1896,62 @@ template <class T>
 int fwd_scalar(OraclePlan* p, const T* f, cudaStream_t st) {
   using C = cplx<T>;
   const GridK g = p->g;
-  { Launch L_(p, 0, st); k_fx<T, FX_FIELDS><<<grid_x(p, p->zc_fx), kFftThreads, smem_fx(p, 2), st>>>(
-      g, p->pxf, p->zc_fx, 1, f, nullptr, nullptr, nullptr, 0.0, p->rho, p->rhoh, p->theta0,
-      p->kx, (const C*)p->twx, (C*)p->S1, nullptr, nullptr); }
-  OB_LAUNCHED();
-  { Launch L_(p, 1, st); k_fy<T, FY_FIELDS><<<grid_y(p, p->zc_fy), kFftThreads, smem_fy(p, 2, p->zc_fy), st>>>(
-      g, p->pyf, p->zc_fy, 1, (C*)p->S1, nullptr, p->kx, p->ky, (const C*)p->twy, 1.0,
-      (C*)p->S3, nullptr); }
-  OB_LAUNCHED();
+  {
+    Launch L_(p, 0, st);
+    if (p->z_fx)
+      OB_CUDA((zfx<T, T>(ZFX_FIELDS, zline_x<T>(p), g, f, nullptr, nullptr, nullptr, 0.0, p->rho,
+                         p->rhoh, (C*)p->S1, nullptr, nullptr, st)));
+    else
+      k_fx<T, FX_FIELDS><<<grid_x(p, p->zc_fx), kFftThreads, smem_fx(p, 2), st>>>(
+          g, p->pxf, p->zc_fx, 1, f, nullptr, nullptr, nullptr, 0.0, p->rho, p->rhoh, p->theta0,
+          p->kx, (const C*)p->twx, (C*)p->S1, nullptr, nullptr);
+    OB_LAUNCHED();
+  }
+  {
+    Launch L_(p, 1, st);
+    if (p->z_fy)
+      OB_CUDA((zfy<T, T>(ZFY_FIELDS, zline_y<T>(p), g, (C*)p->S1, nullptr, nullptr, 0.0, p->kx,
+                         p->ky, (C*)p->S3, nullptr, st)));
+    else
+      k_fy<T, FY_FIELDS><<<grid_y(p, p->zc_fy), kFftThreads, smem_fy(p, 2, p->zc_fy), st>>>(
+          g, p->pyf, p->zc_fy, 1, (C*)p->S1, nullptr, p->kx, p->ky, (const C*)p->twy, 1.0,
+          (C*)p->S3, nullptr);
+    OB_LAUNCHED();
+  }
   return OB_OK;
 }
 
 // inverse 2-D real FFT of S3 (scaled) into out
 template <class T>
 int inv_scalar(OraclePlan* p, double scale, T* out, cudaStream_t st) {
-  using C = cplx<T>;
-  const GridK g = p->g;
-  { Launch L_(p, 3, st); k_iy<T, IY_FIELDS><<<grid_y(p, p->zc_iy), kFftThreads, smem_fy(p, 2, p->zc_iy), st>>>(
-      g, p->py, p->zc_iy, 1, (C*)p->S3, nullptr, p->ky, (const C*)p->twy, scale, (C*)p->S1,
-      nullptr); }
-  OB_LAUNCHED();
-  { Launch L_(p, 4, st); k_ix<T, IX_FIELDS><<<grid_x(p, p->zc_ix), kFftThreads, smem_ix(p, 2 * p->zc_ix), st>>>(
-      g, p->px, p->zc_ix, 1, (C*)p->S1, nullptr, nullptr, p->kx, (const C*)p->twx, nullptr,
-      nullptr, nullptr, nullptr, 0.0, p->theta0, out, nullptr, nullptr, nullptr); }
-  OB_LAUNCHED();
-  return OB_OK;
+  RC(op_iy_field<T>(p, scale, st));
+  return op_ix_field<T>(p, out, st);
 }
 
 template <class T>
 int gradient_impl(OraclePlan* p, const T* phi, T* gx, T* gy, T* gz, cudaStream_t st) {
   using C = cplx<T>;
   const GridK g = p->g;
+  const double scale = 1.0 / ((double)g.nx * (double)g.ny);
   RC(fwd_scalar<T>(p, phi, st));
-  { Launch L_(p, 3, st); k_iy<T, IY_GRAD><<<grid_y(p, p->zc_iy), kFftThreads, smem_fy(p, 2, p->zc_iy), st>>>(
-      g, p->py, p->zc_iy, 2, (C*)p->S3, nullptr, p->ky, (const C*)p->twy,
-      1.0 / ((double)g.nx * (double)g.ny), (C*)p->S1, (C*)p->S2); }
-  OB_LAUNCHED();
-  { Launch L_(p, 4, st); k_ix<T, IX_GRAD><<<grid_x(p, p->zc_ix), kFftThreads, smem_ix(p, 3 * p->zc_ix + 1), st>>>(
-      g, p->px, p->zc_ix, 0, (C*)p->S1, (C*)p->S2, nullptr, p->kx, (const C*)p->twx, nullptr,
-      nullptr, nullptr, nullptr, 0.0, p->theta0, gx, gy, gz, nullptr); }
+  {
+    Launch L_(p, 3, st);
+    if (p->z_iy)
+      OB_CUDA(ziy<T>(true, zline_y<T>(p), g, (C*)p->S3, scale, (C*)p->S1, (C*)p->S2, st));
+    else
+      k_iy<T, IY_GRAD><<<grid_y(p, p->zc_iy), kFftThreads, smem_fy(p, 2, p->zc_iy), st>>>(
+          g, p->py, p->zc_iy, 2, (C*)p->S3, nullptr, p->ky, (const C*)p->twy, scale, (C*)p->S1,
+          (C*)p->S2);
+    OB_LAUNCHED();
+  }
+  Launch L_(p, 4, st);
+  if (p->z_ix)
+    OB_CUDA(zix<T>(ZIX_GRAD, zline_x<T>(p), g, (C*)p->S1, (C*)p->S2, nullptr, nullptr, nullptr,
+                   nullptr, 0.0, gx, gy, gz, nullptr, st));
+  else
+    k_ix<T, IX_GRAD><<<grid_x(p, p->zc_ix), kFftThreads, smem_ix(p, 3 * p->zc_ix + 1), st>>>(
+        g, p->px, p->zc_ix, 0, (C*)p->S1, (C*)p->S2, nullptr, p->kx, (const C*)p->twx, nullptr,
+        nullptr, nullptr, nullptr, 0.0, p->theta0, gx, gy, gz, nullptr);
   OB_LAUNCHED();
   return OB_OK;
 }
@@ -1900,6 +2043,13 @@ int* var_field(OraclePlan* p, int i) {
     case OB_VAR_RZC2_FY: return q ? &q->zc2_fy : nullptr;
     case OB_VAR_ZC4_FYD: return &p->zc4_fyd;
     case OB_VAR_ZC4_FXSH: return &p->zc4_fxsh;
+    case OB_VAR_Z_FX: return &p->z_fx;
+    case OB_VAR_Z_FXS: return &p->z_fxs;
+    case OB_VAR_Z_IX: return &p->z_ix;
+    case OB_VAR_Z_FY: return &p->z_fy;
+    case OB_VAR_Z_IY: return &p->z_iy;
+    case OB_VAR_Z_FXD: return &p->z_fxd;
+    case OB_VAR_Z_FYD: return &p->z_fyd;
   }
   return nullptr;
 }
@@ -1964,6 +2114,13 @@ std::vector<int> var_values(const OraclePlan* p, int i) {
       break;
     case OB_VAR_ZC4_FYD: list(f32 && ny == kY4N && p->dbl, {2}); break;
     case OB_VAR_ZC4_FXSH: list(f32 && p->S4 != nullptr, {2, 4, 8}); break;
+    case OB_VAR_Z_FX:
+    case OB_VAR_Z_FXS:
+    case OB_VAR_Z_IX: list(p->zx_ok, {1}); break;
+    case OB_VAR_Z_FY:
+    case OB_VAR_Z_IY: list(p->zy_ok, {1}); break;
+    case OB_VAR_Z_FXD: list(p->dbl && p->dbl->zx_ok, {1}); break;
+    case OB_VAR_Z_FYD: list(p->dbl && p->dbl->zy_ok, {1}); break;
   }
   return v;
 }
@@ -2040,21 +2197,22 @@ int tune_impl(OraclePlan* p, cudaStream_t st) {
   T *uo = (T*)p->Su, *vo = (T*)p->Sv, *wo = (T*)p->Sw, *po = (T*)p->Sphi;
   const bool stage = p->Bh && p->buoyancy && p->projection;
   const double sdt = 10.0;
-  RC(tune_group<T>(p, {OB_VAR_ZC4_FX, OB_VAR_ZC3_FX, OB_VAR_ZC2_FX}, st,
+  RC(tune_group<T>(p, {OB_VAR_Z_FX, OB_VAR_ZC4_FX, OB_VAR_ZC3_FX, OB_VAR_ZC2_FX}, st,
                    [&] { return proj_fx<T>(p, false, u, v, w, th, nullptr, 0.0, st); }));
   if (stage)
-    RC(tune_group<T>(p, {OB_VAR_ZC4_FXS, OB_VAR_ZC3_FXS, OB_VAR_ZC2_FXS}, st,
+    RC(tune_group<T>(p, {OB_VAR_Z_FXS, OB_VAR_ZC4_FXS, OB_VAR_ZC3_FXS, OB_VAR_ZC2_FXS}, st,
                      [&] { return proj_fx<T>(p, true, u, v, w, th, bh, sdt, st); }));
-  RC(tune_group<T>(p, {OB_VAR_ZC4_IX, OB_VAR_ZC3_IX, OB_VAR_ZC2_IX}, st, [&] {
+  RC(tune_group<T>(p, {OB_VAR_Z_IX, OB_VAR_ZC4_IX, OB_VAR_ZC3_IX, OB_VAR_ZC2_IX}, st, [&] {
     return stage ? proj_ix<T>(p, true, u, v, w, th, bh, sdt, uo, vo, wo, po, st)
                  : proj_ix<T>(p, false, u, v, w, th, nullptr, 0.0, uo, vo, wo, po, st);
   }));
   // forward and inverse y share the 512-point register form's chunk: time
   // the two together for it, and each alone for the others
   {
-    const int fy4 = p->zc4_fy, iy4 = p->zc4_iy;
-    std::vector<std::array<int, 5>> cands;  // zc4_fy, zc4_iy, zc3_fy, zc2_fy, zc2_iy
+    // zc4_fy, zc4_iy, zc3_fy, zc2_fy, zc2_iy
+    std::vector<std::array<int, 5>> cands;
     cands.push_back({0, 0, 0, 0, 0});
+    p->z_fy = p->z_iy = 0;
     auto vals = [&](int i) {
       std::vector<int> r;
       for (int z : var_values(p, i))
@@ -2068,9 +2226,7 @@ int tune_impl(OraclePlan* p, cudaStream_t st) {
     for (int a : y3) cands.push_back({0, 0, a, 0, 0});
     for (int a : f2)
       for (int b : i2) cands.push_back({0, 0, 0, a, b});
-    (void)fy4;
-    (void)iy4;
-    if (cands.size() > 1) {
+    if (cands.size() > 1 || p->zy_ok) {
       // time each forward and inverse form once, then pick the best pair
       auto apply = [&](const std::array<int, 5>& c) {
         p->zc4_fy = c[0];
@@ -2079,18 +2235,27 @@ int tune_impl(OraclePlan* p, cudaStream_t st) {
         p->zc2_fy = c[3];
         p->zc2_iy = c[4];
       };
-      float best = INFINITY;
+      float best = INFINITY, best_f = INFINITY, best_i = INFINITY;
       std::array<int, 5> win = cands[0];
       for (const auto& c : cands) {
         apply(c);
-        const float t = time_launch(st, [&] { return proj_fy<T>(p, st); }) +
-                        time_launch(st, [&] { return proj_iy<T>(p, 3, st); });
-        if (t < best) {
-          best = t;
+        const float f = time_launch(st, [&] { return proj_fy<T>(p, st); });
+        const float i = time_launch(st, [&] { return proj_iy<T>(p, 3, st); });
+        if (f + i < best) {
+          best = f + i;
+          best_f = f;
+          best_i = i;
           win = c;
         }
       }
       apply(win);
+      // the level-paired lines, each way alone
+      if (p->zy_ok) {
+        p->z_fy = 1;
+        p->z_fy = time_launch(st, [&] { return proj_fy<T>(p, st); }) < best_f;
+        p->z_iy = 1;
+        p->z_iy = time_launch(st, [&] { return proj_iy<T>(p, 3, st); }) < best_i;
+      }
     }
   }
   if constexpr (sizeof(T) == 4) {
@@ -2098,10 +2263,10 @@ int tune_impl(OraclePlan* p, cudaStream_t st) {
       return thomas_solve<T>(p, 2, (cplx<T>*)p->S3, nullptr, 0, 0, st);
     }));
     if (p->dbl) {
-      RC(tune_group<T>(p, {OB_VAR_ZC4_FXD, OB_VAR_ZC3_FXD, OB_VAR_RZC2_FX}, st,
+      RC(tune_group<T>(p, {OB_VAR_Z_FXD, OB_VAR_ZC4_FXD, OB_VAR_ZC3_FXD, OB_VAR_RZC2_FX}, st,
                        [&] { return refine_fx(p, (const float*)u, (const float*)v,
                                               (const float*)w, st); }));
-      RC(tune_group<T>(p, {OB_VAR_ZC4_FYD, OB_VAR_ZC3_FYD, OB_VAR_RZC2_FY}, st,
+      RC(tune_group<T>(p, {OB_VAR_Z_FYD, OB_VAR_ZC4_FYD, OB_VAR_ZC3_FYD, OB_VAR_RZC2_FY}, st,
                        [&] { return refine_fy(p, st); }));
     }
     const bool slow = p->advection || p->coriolis || p->heating;
@@ -2148,7 +2313,7 @@ std::string tune_key(const OraclePlan* p) {
   cudaDeviceProp prop{};
   cudaGetDeviceProperties(&prop, dev);
   char buf[512];
-  snprintf(buf, sizeof buf, "v1 %dx%dx%d prec%d stage%d slow%d%d%d%d prod%d%d%d%d damp%d sm%d %s",
+  snprintf(buf, sizeof buf, "v2 %dx%dx%d prec%d stage%d slow%d%d%d%d prod%d%d%d%d damp%d sm%d %s",
            p->g.nx, p->g.ny, p->g.nz, p->prec, (int)(p->buoyancy && p->projection),
            p->advection, p->coriolis, p->heating, p->damping, p->drag, p->sponge, p->diffusion,
            p->cooling, p->damping, nsm, prop.name);
@@ -2813,6 +2978,12 @@ int oracle_b200_plan_create(const OracleGridDesc* grid, const OracleComponentDes
     }
   }
 
+  if ((rc = p->prec == OB_PREC_F64 ? make_zlines<double>(p, p, kx.data(), ky.data())
+                                   : make_zlines<float>(p, p, kx.data(), ky.data())))
+    return bail(rc);
+  p->z_fx = p->z_fxs = p->z_ix = p->zx_ok;
+  p->z_fy = p->z_iy = p->zy_ok;
+
   const size_t n = (size_t)nx * ny * nz, nw = (size_t)nx * ny * (nz + 1);
   const size_t ns = (size_t)p->g.nxh * ny * nz;
   const size_t e = p->esz;
@@ -2878,7 +3049,7 @@ int oracle_b200_plan_create(const OracleGridDesc* grid, const OracleComponentDes
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   p->nparts = nsm * 4;
   if ((rc = dalloc(p, &p->parts, p->nparts * sizeof(DiagPart)))) return bail(rc);
-  if (p->prec == OB_PREC_F32 && (rc = make_refiner(p))) return bail(rc);
+  if (p->prec == OB_PREC_F32 && (rc = make_refiner(p, kx.data(), ky.data()))) return bail(rc);
   // allocations and table copies complete: the memory is usable on any stream
   if (cudaStreamSynchronize(p->astream) != cudaSuccess)
     return bail(fail(OB_ERR_CUDA, "plan_create: set-up stream failed"));

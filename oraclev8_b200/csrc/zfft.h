@@ -1,0 +1,75 @@
+// Host interface of the level-paired line transforms (zfft.cuh): line plans and
+// launchers, compiled apart from the C ABI (zfft.cu, once per precision).
+#pragma once
+#include "common.cuh"
+
+namespace ob {
+
+// A line's factorisation N = r[0] r[1] .. r[np-1].  Position of the digit
+// vector (j0, j1, ..): j0 + S[1] j1 + S[2] j2 + ..; it holds input row
+// n = j_last + r_last (j_prev + ..) before a forward transform and wavenumber
+// j0 + S[1] j1 + .. after it.
+struct ZPlan {
+  int N, np, Q;     // Q = N / r[np-1]: stride of the last forward pass
+  int r[4], S[4];   // radix and stride of each forward pass
+  int nb[4];        // butterflies per line N / r[i]
+  int sh, NP;       // pad shift, padded length
+  int ns;           // butterfly pairs (t, Q - t) of the last forward pass
+  FastDiv dS[4], dnb[4], dr[4], dns;
+};
+
+// The plan of an even line of N points with elements of `elem` bytes (4 or 8);
+// false where N has no factorisation in the kernels' radices or two buffers of
+// one line exceed shared memory.
+bool zplan_make(int N, int elem, ZPlan* out);
+
+// The index into W_N^t of every entry of the line's pass twiddles (N entries).
+void zplan_twiddles(const ZPlan& p, int* t);
+
+// One direction's lines: plan and device tables.
+template <class T>
+struct ZLine {
+  ZPlan plan;
+  const T* k;          // wavenumbers, the Nyquist entry zeroed
+  const cplx<T>* tw;   // pass twiddles (zplan_twiddles)
+};
+
+// forward x modes
+#define ZFX_DIV 0     // X0 = i kx' F(rho u) + F(D w), X1 = F(rho v)
+#define ZFX_STAGE 1   // the same of w + sdt b_half
+#define ZFX_SHARED 2  // ZFX_DIV and X2 = F(D b_half)
+#define ZFX_FIELDS 3  // X0 = F(u), X1 = F(v) (v null: X0 alone)
+// inverse x modes
+#define ZIX_CORRECT 0  // u, v, w -= grad phi; phi stored unless null
+#define ZIX_STAGE 1    // out = (u, v, w + sdt b_half) - grad phi
+#define ZIX_REFINE 2   // ZIX_CORRECT with phi += the line
+#define ZIX_FIELDS 3   // uo = F^-1(S1), vo = F^-1(S2) (S2 null: uo alone)
+#define ZIX_GRAD 4     // uo, vo, wo = the gradient (wo on nz + 1 levels, 0 at the ends)
+// forward y modes
+#define ZFY_DIV 0     // out0 = F(X0) + i ky' F(X1)
+#define ZFY_SHARED 1  // out0 = F(X0 + s X2) + i ky' F(X1): a fast stage
+#define ZFY_RESID 2   // ZFY_DIV, zero on the Nyquist rows, rounded to TO
+#define ZFY_FIELDS 3  // out0 = F(X0)
+#define ZFY_HELM 4    // forward, the damper's multipliers (times s), and back
+
+// Raises the kernels' shared-memory limits on the current device.
+template <class T>
+cudaError_t zfft_init();
+
+template <class T, class TS>
+cudaError_t zfx(int mode, const ZLine<T>& l, const GridK& g, const TS* u, const TS* v,
+                const TS* w, const TS* bh, double sdt, const double* rho, const double* rhoh,
+                cplx<T>* X0, cplx<T>* X1, cplx<T>* X2, cudaStream_t st);
+template <class T>
+cudaError_t zix(int mode, const ZLine<T>& l, const GridK& g, const cplx<T>* S1,
+                const cplx<T>* S2, const T* u, const T* v, const T* w, const T* bh, double sdt,
+                T* uo, T* vo, T* wo, T* phio, cudaStream_t st);
+template <class T, class TO>
+cudaError_t zfy(int mode, const ZLine<T>& l, const GridK& g, const cplx<T>* X0,
+                const cplx<T>* X1, const cplx<T>* X2, double s, const double* kxd,
+                const double* kyd, cplx<TO>* out0, cplx<T>* out1, cudaStream_t st);
+template <class T>
+cudaError_t ziy(bool grad, const ZLine<T>& l, const GridK& g, const cplx<T>* in, double scale,
+                cplx<T>* out0, cplx<T>* out1, cudaStream_t st);
+
+}  // namespace ob
