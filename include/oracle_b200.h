@@ -137,7 +137,9 @@ extern "C" {
 #define OB_VAR_Z_IY 27
 #define OB_VAR_Z_FXD 28
 #define OB_VAR_Z_FYD 29
-#define OB_VAR_COUNT 30
+#define OB_VAR_Z_YZ 30  /* forward y, the vertical solve and inverse y in one launch, a kx
+                         * plane per block (planes that fit shared memory) */
+#define OB_VAR_COUNT 31
 
 #define OB_TUNE_FORCE 1  /* time the candidates even when a choice is cached */
 
@@ -492,7 +494,7 @@ const char *oracle_b200_last_error(void);
  * that bindings can refuse a library built from another header.  2: the
  * shared stage transforms (OB_VAR_ZC4_FXSH, OB_VAR_COUNT 23) and the
  * long-wave Thomas profile class (OB_PROF_THOMAS_LW, OB_PROF_CLASSES 10).  3:
- * the level-paired line transforms (OB_VAR_Z_*, OB_VAR_COUNT 30). */
+ * the level-paired line transforms (OB_VAR_Z_*, OB_VAR_COUNT 31). */
 #define OB_ABI_VERSION 3
 int oracle_b200_version(void);
 

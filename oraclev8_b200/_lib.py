@@ -46,7 +46,8 @@ EXPORTS = (
 VARIANTS = ("zc2_fx", "zc2_fxs", "zc2_ix", "zc2_fy", "zc2_iy", "zc3_fx", "zc3_fxs", "zc3_ix",
             "zc3_fxd", "zc3_fy", "zc3_fyd", "zc4_fx", "zc4_fxs", "zc4_ix", "zc4_fxd", "zc4_fy",
             "zc4_iy", "slow_xw", "thomas_fast", "rzc2_fx", "rzc2_fy", "zc4_fyd", "zc4_fxsh", "z_fx",
-            "z_fxs", "z_ix", "z_fy", "z_iy", "z_fxd", "z_fyd")
+            "z_fxs", "z_ix", "z_fy", "z_iy", "z_fxd", "z_fyd",
+            "z_yz")
 OB_TUNE_FORCE = 1
 ABI_VERSION = 3  # OB_ABI_VERSION of the header these tables follow
 PROF_CLASSES = ("fx", "fy", "thomas", "iy", "ix", "slow", "diag", "other", "refine",

@@ -240,6 +240,9 @@ struct OraclePlan {
   bool zx_ok = false, zy_ok = false;
   void *zkx = nullptr, *zky = nullptr, *ztx = nullptr, *zty = nullptr;
   int z_fx = 0, z_fxs = 0, z_ix = 0, z_fy = 0, z_iy = 0, z_fxd = 0, z_fyd = 0;
+  // the plane form of y, solve and y back (zplane.cuh) and its reciprocal pivots
+  int z_yz = 0;
+  double* zinv = nullptr;
   // FP32 slow tendency: 0 the gather form, 1 marching along x (k_slow_xw),
   // 4 / 8 marching along x over bulk-copied planes of 4 / 8 rows (k_slow_xt)
   int slow_xw = 1;
@@ -1119,6 +1122,38 @@ int thomas_solve(OraclePlan* p, int cls, cplx<T>* S3, double* diag, int slot_c, 
   return OB_OK;
 }
 
+// The plane form's tables; empty where a plane does not fit shared memory.
+ZSolve zsolve_args(const OraclePlan* p) {
+  return {p->zinv, p->dbl ? (cplx<double>*)p->dbl->S1 : nullptr, p->lw_flag};
+}
+template <class T>
+int make_zsolve(OraclePlan* p) {
+  if (!p->zy_ok || !zplane_group<T>(p->zpy, p->g.nz)) return OB_OK;
+  RC(dalloc(p, &p->zinv, (size_t)p->g.nxh * p->g.ny * p->g.nz * sizeof(double)));
+  OB_CUDA(zplane_inv(p->g, thomas_args(p), p->zinv, p->astream));
+  return OB_OK;
+}
+
+// The residuals of a solve that logs them, where its solution comes from the
+// plane form: the generic sweeps in place on S3, whose result nothing reads.
+template <class T>
+int thomas_residuals(OraclePlan* p, double* diag, int slot_c, int slot_d, cudaStream_t st) {
+  const long ncols = (long)p->g.nxh * p->g.ny;
+  const unsigned nb = (unsigned)((ncols + kThomasCols - 1) / kThomasCols);
+  cplx<T>* S3 = (cplx<T>*)p->S3;
+  if (sizeof(T) == 8 || !p->lw_blocks) {
+    { Launch L_(p, 2, st); k_thomas<T, kThomasCols><<<nb, kThomasCols, smem_thomas(p), st>>>(
+          p->g, thomas_args(p), S3, S3, diag, slot_c, slot_d); }
+  } else {
+    { Launch L_(p, 2, st); k_thomas<T, kThomasCols, double><<<(unsigned)p->n_lw, kThomasCols, smem_thomas(p, 8), st>>>(
+          p->g, thomas_args(p), S3, S3, diag, slot_c, slot_d, p->lw_blocks, nullptr); }
+    { Launch L_(p, 2, st); k_thomas<T, kThomasCols, float><<<nb, kThomasCols, smem_thomas(p, 4), st>>>(
+          p->g, thomas_args(p), S3, S3, diag, slot_c, slot_d, nullptr, p->lw_flag); }
+  }
+  OB_LAUNCHED();
+  return OB_OK;
+}
+
 // ---- projection pipeline -------------------------------------------------
 // One launcher per kernel class of the projection; each runs the variant the
 // plan's choice fields select (register-resident > compile-time-chunk pencils
@@ -1230,6 +1265,17 @@ int proj_iy(OraclePlan* p, int cls, cudaStream_t st) {
   return OB_OK;
 }
 
+// the plane form: forward y of (X0, X1) (or their spectrum itself), the solve
+// and inverse y into (S1, out1), in place
+template <class T>
+int proj_yz(OraclePlan* p, int cls, bool fwd, const cplx<T>* X0, const cplx<T>* X1, cplx<T>* out1,
+            cudaStream_t st) {
+  Launch L_(p, cls, st);
+  OB_CUDA(zplane<T>(zline_y<T>(p), p->g, thomas_args(p), zsolve_args(p), fwd, X0, X1,
+                    (cplx<T>*)p->S1, out1, st));
+  return OB_OK;
+}
+
 // inverse x with the velocity correction: (S1, S2) and the state -> outputs
 template <class T>
 int proj_ix(OraclePlan* p, bool stage, const T* u, const T* v, const T* w, const T* th,
@@ -1308,6 +1354,14 @@ int project_impl(OraclePlan* p, const T* u, const T* v, const T* w, const T* th,
     OB_LAUNCHED();
   } else {
     RC(proj_fx<T>(p, stage, u, v, w, th, bh, stage_sdt, st));
+    if (p->z_yz) {
+      if (diag) {
+        RC(proj_fy<T>(p, st));
+        RC(thomas_residuals<T>(p, diag, slot_c, slot_d, st));
+      }
+      RC(proj_yz<T>(p, 2, true, (cplx<T>*)p->S1, (cplx<T>*)p->S2, (cplx<T>*)p->S2, st));
+      return proj_ix<T>(p, stage, u, v, w, th, bh, stage_sdt, uo, vo, wo, phio, st);
+    }
     RC(proj_fy<T>(p, st));
   }
   RC(thomas_solve<T>(p, 2, (cplx<T>*)p->S3, diag, slot_c, slot_d, st));
@@ -1392,8 +1446,12 @@ int refine_impl(OraclePlan* p, float* u, float* v, float* w, float* phi, cudaStr
   Cf* S3 = (Cf*)p->S3;
   RC(refine_fx(p, u, v, w, st));
   RC(refine_fy(p, st));
-  RC(thomas_solve<float>(p, OB_PROF_REFINE, S3, nullptr, 0, 0, st));
-  RC(proj_iy<float>(p, OB_PROF_REFINE, st));
+  if (p->z_yz) {
+    RC(proj_yz<float>(p, OB_PROF_REFINE, false, S3, nullptr, S2, st));
+  } else {
+    RC(thomas_solve<float>(p, OB_PROF_REFINE, S3, nullptr, 0, 0, st));
+    RC(proj_iy<float>(p, OB_PROF_REFINE, st));
+  }
   if (p->z_ix) {
     Launch L_(p, OB_PROF_REFINE, st);
     OB_CUDA(zix<float>(ZIX_REFINE, zline_x<float>(p), g, S1, S2, u, v, w, nullptr, 0.0, u, v, w,
@@ -1891,22 +1949,28 @@ int divergence_impl(OraclePlan* p, const T* u, const T* v, const T* w, T* d, cud
   return op_ix_field<T>(p, d, st);
 }
 
+// forward x FFT of one field into S1
+template <class T>
+int fwd_x(OraclePlan* p, const T* f, cudaStream_t st) {
+  using C = cplx<T>;
+  Launch L_(p, 0, st);
+  if (p->z_fx)
+    OB_CUDA((zfx<T, T>(ZFX_FIELDS, zline_x<T>(p), p->g, f, nullptr, nullptr, nullptr, 0.0, p->rho,
+                       p->rhoh, (C*)p->S1, nullptr, nullptr, st)));
+  else
+    k_fx<T, FX_FIELDS><<<grid_x(p, p->zc_fx), kFftThreads, smem_fx(p, 2), st>>>(
+        p->g, p->pxf, p->zc_fx, 1, f, nullptr, nullptr, nullptr, 0.0, p->rho, p->rhoh, p->theta0,
+        p->kx, (const C*)p->twx, (C*)p->S1, nullptr, nullptr);
+  OB_LAUNCHED();
+  return OB_OK;
+}
+
 // forward 2-D real FFT of one field into S3 (unnormalised)
 template <class T>
 int fwd_scalar(OraclePlan* p, const T* f, cudaStream_t st) {
   using C = cplx<T>;
   const GridK g = p->g;
-  {
-    Launch L_(p, 0, st);
-    if (p->z_fx)
-      OB_CUDA((zfx<T, T>(ZFX_FIELDS, zline_x<T>(p), g, f, nullptr, nullptr, nullptr, 0.0, p->rho,
-                         p->rhoh, (C*)p->S1, nullptr, nullptr, st)));
-    else
-      k_fx<T, FX_FIELDS><<<grid_x(p, p->zc_fx), kFftThreads, smem_fx(p, 2), st>>>(
-          g, p->pxf, p->zc_fx, 1, f, nullptr, nullptr, nullptr, 0.0, p->rho, p->rhoh, p->theta0,
-          p->kx, (const C*)p->twx, (C*)p->S1, nullptr, nullptr);
-    OB_LAUNCHED();
-  }
+  RC(fwd_x<T>(p, f, st));
   {
     Launch L_(p, 1, st);
     if (p->z_fy)
@@ -1960,6 +2024,11 @@ template <class T>
 int solve_impl(OraclePlan* p, const T* d, T* phi, int log_diag, cudaStream_t st) {
   using C = cplx<T>;
   const GridK g = p->g;
+  if (sizeof(T) == 8 && p->z_yz && !log_diag) {  // FP32 plans solve every column in double here
+    RC(fwd_x<T>(p, d, st));
+    RC(proj_yz<T>(p, 2, true, (C*)p->S1, nullptr, nullptr, st));
+    return op_ix_field<T>(p, phi, st);
+  }
   RC(fwd_scalar<T>(p, d, st));
   double* diag = nullptr;
   if (log_diag) {
@@ -2050,6 +2119,7 @@ int* var_field(OraclePlan* p, int i) {
     case OB_VAR_Z_IY: return &p->z_iy;
     case OB_VAR_Z_FXD: return &p->z_fxd;
     case OB_VAR_Z_FYD: return &p->z_fyd;
+    case OB_VAR_Z_YZ: return &p->z_yz;
   }
   return nullptr;
 }
@@ -2121,6 +2191,7 @@ std::vector<int> var_values(const OraclePlan* p, int i) {
     case OB_VAR_Z_IY: list(p->zy_ok, {1}); break;
     case OB_VAR_Z_FXD: list(p->dbl && p->dbl->zx_ok, {1}); break;
     case OB_VAR_Z_FYD: list(p->dbl && p->dbl->zy_ok, {1}); break;
+    case OB_VAR_Z_YZ: list(p->zinv != nullptr, {1}); break;
   }
   return v;
 }
@@ -2262,6 +2333,16 @@ int tune_impl(OraclePlan* p, cudaStream_t st) {
     RC(tune_group<T>(p, {OB_VAR_THOMAS_FAST}, st, [&] {
       return thomas_solve<T>(p, 2, (cplx<T>*)p->S3, nullptr, 0, 0, st);
     }));
+  }
+  // y, solve and y back in one launch against their three
+  RC(tune_group<T>(p, {OB_VAR_Z_YZ}, st, [&] {
+    if (p->z_yz)
+      return proj_yz<T>(p, 2, true, (cplx<T>*)p->S1, (cplx<T>*)p->S2, (cplx<T>*)p->S2, st);
+    RC(proj_fy<T>(p, st));
+    RC(thomas_solve<T>(p, 2, (cplx<T>*)p->S3, nullptr, 0, 0, st));
+    return proj_iy<T>(p, 3, st);
+  }));
+  if constexpr (sizeof(T) == 4) {
     if (p->dbl) {
       RC(tune_group<T>(p, {OB_VAR_Z_FXD, OB_VAR_ZC4_FXD, OB_VAR_ZC3_FXD, OB_VAR_RZC2_FX}, st,
                        [&] { return refine_fx(p, (const float*)u, (const float*)v,
@@ -2313,7 +2394,7 @@ std::string tune_key(const OraclePlan* p) {
   cudaDeviceProp prop{};
   cudaGetDeviceProperties(&prop, dev);
   char buf[512];
-  snprintf(buf, sizeof buf, "v2 %dx%dx%d prec%d stage%d slow%d%d%d%d prod%d%d%d%d damp%d sm%d %s",
+  snprintf(buf, sizeof buf, "v3 %dx%dx%d prec%d stage%d slow%d%d%d%d prod%d%d%d%d damp%d sm%d %s",
            p->g.nx, p->g.ny, p->g.nz, p->prec, (int)(p->buoyancy && p->projection),
            p->advection, p->coriolis, p->heating, p->damping, p->drag, p->sponge, p->diffusion,
            p->cooling, p->damping, nsm, prop.name);
@@ -3050,6 +3131,9 @@ int oracle_b200_plan_create(const OracleGridDesc* grid, const OracleComponentDes
   p->nparts = nsm * 4;
   if ((rc = dalloc(p, &p->parts, p->nparts * sizeof(DiagPart)))) return bail(rc);
   if (p->prec == OB_PREC_F32 && (rc = make_refiner(p, kx.data(), ky.data()))) return bail(rc);
+  if ((rc = p->prec == OB_PREC_F64 ? make_zsolve<double>(p) : make_zsolve<float>(p)))
+    return bail(rc);
+  p->z_yz = p->zinv != nullptr;
   // allocations and table copies complete: the memory is usable on any stream
   if (cudaStreamSynchronize(p->astream) != cudaSuccess)
     return bail(fail(OB_ERR_CUDA, "plan_create: set-up stream failed"));

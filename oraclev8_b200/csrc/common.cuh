@@ -103,6 +103,23 @@ struct FftPlan {
   FastDiv ns[16];
 };
 
+// Thomas tables (double, device), built on the host exactly as
+// poisson.py:286-325 builds them.
+struct ThomasK {
+  const double* a;     // (nz) sub-diagonal, a[0] = 0
+  const double* c;     // (nz) super-diagonal, c[nz-1] = 0
+  const double* negs;  // (nz) mode-independent part of the diagonal
+  const double* rho;   // (nz) rho on full levels (multiplies k^2)
+  const double* rhoh;  // (nz+1) rho on half levels (residual operator)
+  const double* kx;    // (nx) 2 pi fftfreq
+  const double* ky;    // (ny)
+  const double* a0;    // (nz-1) zero-mode reduced system
+  const double* cp0;
+  const double* inv0;
+  double dz;
+  double scale;        // 1 / (nx ny): inverse-FFT normalisation folded in
+};
+
 constexpr double kGravity = 9.81;  // oracle_v8/constants.py:25
 
 }  // namespace ob

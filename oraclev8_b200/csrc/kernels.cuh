@@ -264,23 +264,6 @@ __global__ void __launch_bounds__(256, 2) k_fy(GridK g, FftPlan py, int zc, int 
   }
 }
 
-// Thomas tables (double, device), built on the host exactly as
-// poisson.py:286-325 builds them.
-struct ThomasK {
-  const double* a;     // (nz) sub-diagonal, a[0] = 0
-  const double* c;     // (nz) super-diagonal, c[nz-1] = 0
-  const double* negs;  // (nz) mode-independent part of the diagonal
-  const double* rho;   // (nz) rho on full levels (multiplies k^2)
-  const double* rhoh;  // (nz+1) rho on half levels (residual operator)
-  const double* kx;    // (nx) 2 pi fftfreq
-  const double* ky;    // (ny)
-  const double* a0;    // (nz-1) zero-mode reduced system
-  const double* cp0;
-  const double* inv0;
-  double dz;
-  double scale;        // 1 / (nx ny): inverse-FFT normalisation folded in
-};
-
 // Byte offset of a k_thomas CTA's staged columns: after the zero-mode region
 // (3 P doubles), rounded up to 16 bytes for the cp.async copies.
 __host__ __device__ inline size_t thomas_stage_offset(int P) {

@@ -6,12 +6,16 @@
 #include <cstdlib>
 
 #include "zfft.cuh"
+#if OB_ZPART == 0
+#include "zplane.cuh"
+#endif
 
 namespace ob {
 
 namespace {
 
 constexpr size_t kZSmemMax = 227 * 1024;
+constexpr size_t kZSmemShare = 176 * 1024;
 constexpr long kZFill = 2 * 148;  // CTAs below which lines are not batched
 
 // Lines per CTA and threads: at least 128 threads' worth of radix-8
@@ -33,6 +37,13 @@ Shape shape(const ZPlan& p, int C, int nbuf, int lines, int chunks, int most) {
   s.threads = std::min(most, std::max(64, (rows * per + 31) / 32 * 32));
   s.grid = dim3(chunks, (lines + rows - 1) / rows);
   s.smem = (size_t)nbuf * rows * p.NP * C * 2 * sizeof(T);
+  // Where the resident blocks' lines would take most of the SM's memory, one
+  // block fewer leaves the first-level cache room for the rows' neighbouring
+  // accesses (1024 points, single precision: forward y 456 -> 372 us): ask for
+  // enough that it does not fit.
+  const size_t resident = std::min<size_t>(65536 / ((sizeof(T) == 4 ? 80 : 128) * s.threads),
+                                           kZSmemMax / s.smem);
+  if (resident > 2 && resident * s.smem > kZSmemShare) s.smem = kZSmemMax / resident + 1024;
   return s;
 }
 
@@ -90,7 +101,8 @@ cudaError_t zfx_last(int mode, const ZLine<T>& l, const GridK& g, const TS* u, c
                      const double* rhoh, cplx<T>* X0, cplx<T>* X1, cplx<T>* X2,
                      cudaStream_t st) {
   constexpr int C = zx_pairs<T>();
-  const Shape s = shape<T>(l.plan, C, 1, g.ny, div_up(g.nz, 2 * C), zx_threads<T>());
+  const int sets = mode == ZFX_FIELDS && !v ? 1 : mode == ZFX_SHARED ? 3 : 2;
+  const Shape s = shape<T>(l.plan, C, 1, g.ny, sets * div_up(g.nz, 2 * C), zx_threads<T>());
 #define OB_ZFX(M)                                                                              \
   case M:                                                                                      \
     k_zfx<T, TS, M, RL><<<s.grid, s.threads, s.smem, st>>>(l.plan, g, s.rows, u, v, w, bh, sdt, \
@@ -116,7 +128,11 @@ cudaError_t zix_last(int mode, const ZLine<T>& l, const GridK& g, const cplx<T>*
                      const cplx<T>* S2, const T* u, const T* v, const T* w, const T* bh,
                      double sdt, T* uo, T* vo, T* wo, T* phio, cudaStream_t st) {
   constexpr int C = zx_pairs<T>();
-  const Shape s = shape<T>(l.plan, C, 1, g.ny, div_up(g.nz, 2 * C), zx_threads<T>());
+  const int chunks = div_up(g.nz, 2 * C);
+  const int blocks = mode == ZIX_FIELDS ? (S2 ? 2 : 1) * chunks
+                     : mode != ZIX_GRAD && phio ? 2 * chunks + div_up(g.nz, 2 * C - 1)
+                                                : 3 * chunks;
+  const Shape s = shape<T>(l.plan, C, 1, g.ny, blocks, zx_threads<T>());
 #define OB_ZIX(M)                                                                               \
   case M:                                                                                       \
     k_zix<T, T, M, RL><<<s.grid, s.threads, s.smem, st>>>(l.plan, g, s.rows, S1, S2, l.k, l.tw, \
@@ -165,6 +181,7 @@ cudaError_t zfft_init<T>() {
   OB_Z(attr(k_zfy2<T, T, ZFY_HELM, C / 2>));
   OB_Z(attr(k_ziy<T, true>));
   OB_Z(attr(k_ziy<T, false>));
+  OB_Z(attr(k_zplane<T>));
 #if OB_ZWIDE
   OB_Z(attr(k_zfy2<T, float, ZFY_RESID, C>));
   OB_Z(attr(k_zfy2<T, float, ZFY_RESID, C / 2>));
@@ -254,6 +271,39 @@ cudaError_t ziy(bool grad, const ZLine<T>& l, const GridK& g, const cplx<T>* in,
                                                        out0, out1);
   return cudaGetLastError();
 }
+
+template <>
+int zplane_group<T>(const ZPlan& p, int nz) {
+  const int C = zy_cols<T>(), nch = div_up(nz, C);
+  int best = 0;
+  for (int q = 1; q <= nch; ++q)
+    if (zplane_layout<T>(p.NP, nz, q).total <= kZSmemMax) best = q;
+  // groups of even size: as few as the largest one gives
+  return best ? div_up(nch, div_up(nch, best)) : 0;
+}
+
+template <>
+cudaError_t zplane<T>(const ZLine<T>& l, const GridK& g, const ThomasK& t, const ZSolve& s,
+                      bool fwd, const cplx<T>* X0, const cplx<T>* X1, cplx<T>* out0, cplx<T>* out1,
+                      cudaStream_t st) {
+  const int group = zplane_group<T>(l.plan, g.nz);
+  if (!group) return cudaErrorInvalidValue;
+  const size_t smem = zplane_layout<T>(l.plan.NP, g.nz, group).total;
+  const int per = l.plan.N * div_up(g.nz, zy_cols<T>()) * zy_cols<T>() / 8;
+  // a warp more than the columns fill, for the zero mode, where that costs none
+  const int threads = std::min(kZPlaneThreads,
+                               std::max({128, div_up(per, 64) * 64, div_up(g.ny, 32) * 32 + 32}));
+  k_zplane<T><<<g.nxh, threads, smem, st>>>(l.plan, g, group, fwd, X0, X1, l.k, l.tw, t, s.inv,
+                                            s.dpd, s.lw, out0, out1);
+  return cudaGetLastError();
+}
+
+#if OB_ZWIDE
+cudaError_t zplane_inv(const GridK& g, const ThomasK& t, double* inv, cudaStream_t st) {
+  k_zinv<<<div_up(g.nxh * g.ny, 128), 128, 0, st>>>(g, t, inv);
+  return cudaGetLastError();
+}
+#endif
 
 #define OB_ZFX_INST(TS)                                                                      \
   template cudaError_t zfx<T, TS>(int, const ZLine<T>&, const GridK&, const TS*, const TS*,  \

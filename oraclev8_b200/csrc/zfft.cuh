@@ -21,10 +21,10 @@
 // loads and barriers at the 16 warps per SM their registers allow; at small
 // grids the latency of the three passes.  Measured per launch against the best
 // earlier form (device time, us):
-//   512 x 512 x 64 double:    x 474 -> 273 and back 551 -> 378, y 186 -> 117
+//   512 x 512 x 64 double:    x 474 -> 246 and back 551 -> 350, y 186 -> 117
 //                             and back 203 -> 127
-//   1024 x 1024 x 80 single:  x back 1600 -> 1030
-//   512 x 512 x 64 single:    x back 261 -> 200
+//   1024 x 1024 x 80 single:  x back 1600 -> 1040, y 428 -> 372 and back 376 -> 340
+//   512 x 512 x 64 single:    x 158 -> 135 and back 261 -> 172
 //
 // Lanes: consecutive threads take consecutive columns (level pairs, or levels
 // in the y kernels), then consecutive butterflies of a line.  Positions in the
@@ -193,15 +193,18 @@ __device__ __forceinline__ cplx<T> ztw(cplx<T> a, const cplx<T>* __restrict__ tw
 }
 
 // A pass between the first and the last, in place (forward: twiddles before
-// the DFT; inverse: after it).  buf: RY lines of NP slots of C columns.
+// the DFT; inverse: after it).  buf: RY lines of NP slots of C columns, slots st
+// and lines rs elements apart (by default packed).
 template <class T, int C, bool INV>
 __device__ __forceinline__ void z_mid_pass(const ZPlan& p, int i, cplx<T>* buf, int RY,
-                                           const cplx<T>* __restrict__ tw) {
+                                           const cplx<T>* __restrict__ tw, int st = C,
+                                           int rs = 0) {
+  if (!rs) rs = p.NP * C;
   constexpr int LC = zlog2(C);
   z_mid(p.r[i], [&](auto rc) {
     constexpr int R = decltype(rc)::value;
     const int S = p.S[i], nb = p.nb[i];
-    const int Sp = (S + (S >> p.sh)) * C;
+    const int Sp = (S + (S >> p.sh)) * st;
     const int tot = RY * nb * C;
     for (int e = ztid(); e < tot; e += blockDim.x) {
       const int c = e & (C - 1);
@@ -212,7 +215,7 @@ __device__ __forceinline__ void z_mid_pass(const ZPlan& p, int i, cplx<T>* buf, 
       }
       const int m = p.dS[i].div(b);
       const int k = b - m * S;
-      cplx<T>* q = buf + ((size_t)row * p.NP + zphys(p, m * (S * R) + k)) * C + c;
+      cplx<T>* q = buf + row * rs + zphys(p, m * (S * R) + k) * st + c;
       cplx<T> v[R];
 #pragma unroll
       for (int j = 0; j < R; ++j) v[j] = q[j * Sp];
@@ -235,7 +238,9 @@ __device__ __forceinline__ void z_mid_pass(const ZPlan& p, int i, cplx<T>* buf, 
 // The adjacent-position pass of a forward transform: load(row, c, n, v) gives
 // the butterfly's inputs of rows n, n + N / R, ..
 template <class T, int C, class Load>
-__device__ __forceinline__ void z_first_fwd(const ZPlan& p, cplx<T>* buf, int RY, Load&& load) {
+__device__ __forceinline__ void z_first_fwd(const ZPlan& p, cplx<T>* buf, int RY, Load&& load,
+                                            int st = C, int rs = 0) {
+  if (!rs) rs = p.NP * C;
   constexpr int LC = zlog2(C);
   z_edge(p.r[0], [&](auto rc) {
     constexpr int R = decltype(rc)::value;
@@ -251,9 +256,9 @@ __device__ __forceinline__ void z_first_fwd(const ZPlan& p, cplx<T>* buf, int RY
       cplx<T> v[R];
       load(rc, row, c, zrev(p, b), nb, v);
       zdft<T, R, false>(v);
-      cplx<T>* q = buf + ((size_t)row * p.NP + zphys(p, b * R)) * C + c;
+      cplx<T>* q = buf + row * rs + zphys(p, b * R) * st + c;
 #pragma unroll
-      for (int j = 0; j < R; ++j) q[j * C] = v[j];
+      for (int j = 0; j < R; ++j) q[j * st] = v[j];
     }
   });
 }
@@ -263,7 +268,8 @@ __device__ __forceinline__ void z_first_fwd(const ZPlan& p, cplx<T>* buf, int RY
 // n, n + step, ..
 template <class T, int C, class Store>
 __device__ __forceinline__ void z_last_inv(const ZPlan& p, const cplx<T>* buf, int RY,
-                                           Store&& store) {
+                                           Store&& store, int st = C, int rs = 0) {
+  if (!rs) rs = p.NP * C;
   constexpr int LC = zlog2(C);
   z_edge(p.r[0], [&](auto rc) {
     constexpr int R = decltype(rc)::value;
@@ -276,8 +282,7 @@ __device__ __forceinline__ void z_last_inv(const ZPlan& p, const cplx<T>* buf, i
         row = p.dnb[0].div(b);
         b -= row * nb;
       }
-      store(rc, row, zrev(p, b), nb,
-            buf + ((size_t)row * p.NP + zphys(p, b * R)) * C + c);
+      store(rc, row, zrev(p, b), nb, buf + row * rs + zphys(p, b * R) * st + c);
     }
   });
 }
@@ -317,7 +322,8 @@ struct cpair {
   cplx<T> a, b;
 };
 template <class T>
-__device__ __forceinline__ cpair<T> ldcpair(const cplx<T>* p, bool vec, bool two) {
+__device__ __forceinline__ cpair<T> ldcpair(const cplx<T>* p, bool vec, bool two,
+                                            bool one = true) {
   cpair<T> r;
   if constexpr (sizeof(T) == 4) {
     if (vec) {
@@ -329,7 +335,7 @@ __device__ __forceinline__ cpair<T> ldcpair(const cplx<T>* p, bool vec, bool two
       return r;
     }
   }
-  r.a = p[0];
+  r.a = one ? p[0] : mk<T>((T)0, (T)0);
   r.b = two ? p[1] : mk<T>((T)0, (T)0);
   return r;
 }
@@ -396,13 +402,14 @@ template <class T>
 __host__ __device__ constexpr int zy_cols() { return sizeof(T) == 4 ? 8 : 4; }
 
 constexpr int kZThreads = 256;
-// threads of an x CTA and CTAs per SM its registers must allow: two paired
-// butterflies, their loads and the column weights take about 120 registers in
-// single precision and 170 in double
+// threads of an x block and blocks per SM its registers must allow: 24 warps of
+// 80 registers in single precision, 16 of 128 in double, some of whose wider
+// butterflies spill; without spills (128 and 168 registers) the fewer warps cost
+// more (512 x 512 x 64, back along x: 194 against 172 us, 362 against 350)
 template <class T>
 __host__ __device__ constexpr int zx_threads() { return sizeof(T) == 4 ? 256 : 128; }
 template <class T>
-__host__ __device__ constexpr int zx_blocks() { return sizeof(T) == 4 ? 2 : 3; }
+__host__ __device__ constexpr int zx_blocks() { return sizeof(T) == 4 ? 3 : 4; }
 
 // Splits the wavenumbers of a paired last pass into the two levels' half
 // spectra and stores them (sum: adds them): v1 = F[t1 + Q j], v2 = F[t2 + Q j],
@@ -454,10 +461,11 @@ __device__ __forceinline__ void z_split_store(const ZPlan& p, int s, bool has2, 
 // stores it with its twiddles.
 template <class T, int R, int C>
 __device__ __forceinline__ void z_first_bfly_inv(const ZPlan& p, cplx<T>* line, int t,
-                                                 const cplx<T>* __restrict__ tw, cplx<T>* x) {
+                                                 const cplx<T>* __restrict__ tw, cplx<T>* x,
+                                                 int st = C) {
   zdft<T, R, true>(x);
-  const int Qp = (p.Q + (p.Q >> p.sh)) * C;
-  cplx<T>* o = line + zphys(p, t) * C;
+  const int Qp = (p.Q + (p.Q >> p.sh)) * st;
+  cplx<T>* o = line + zphys(p, t) * st;
   o[0] = x[0];
 #pragma unroll
   for (int j = 1; j < R; ++j)
@@ -467,9 +475,10 @@ __device__ __forceinline__ void z_first_bfly_inv(const ZPlan& p, cplx<T>* line, 
 // reads and transforms one butterfly of the last forward pass
 template <class T, int R, int C>
 __device__ __forceinline__ void z_last_bfly(const ZPlan& p, const cplx<T>* line, int t,
-                                            const cplx<T>* __restrict__ tw, cplx<T>* v) {
-  const int Qp = (p.Q + (p.Q >> p.sh)) * C;
-  const cplx<T>* q = line + zphys(p, t) * C;
+                                            const cplx<T>* __restrict__ tw, cplx<T>* v,
+                                            int st = C) {
+  const int Qp = (p.Q + (p.Q >> p.sh)) * st;
+  const cplx<T>* q = line + zphys(p, t) * st;
 #pragma unroll
   for (int j = 0; j < R; ++j) v[j] = q[j * Qp];
 #pragma unroll
@@ -493,7 +502,11 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
   cplx<T>* b0 = reinterpret_cast<cplx<T>*>(smem_dyn);
   const int ny = g.ny, nz = g.nz;
   const int y0 = blockIdx.y * RY;
-  const int z = (blockIdx.x * C + (threadIdx.x & (C - 1))) * 2;  // the thread's first level
+  // line sets, a block each: rho u with D w, rho v, the shared form's D b_half
+  constexpr int SETS = MODE == ZFX_SHARED ? 3 : 2;
+  const int sets = MODE == ZFX_FIELDS && !v ? 1 : SETS;
+  const int chunk = blockIdx.x / sets, set = blockIdx.x - chunk * sets;
+  const int z = (chunk * C + (threadIdx.x & (C - 1))) * 2;  // the thread's first level
   const bool on = z < nz, two = z + 1 < nz, vec = !(nz & 1);
   const int rows = min(RY, ny - y0);
   const int xs = ny * nz, ws = ny * (nz + 1);
@@ -550,21 +563,18 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
         r[j] = mk<T>(wdiff(f1, w1[j], f0, w0[j]), two ? wdiff(f2, w2[j], f1, w1[j]) : (T)0);
     };
   };
-  // Runs, one line each: rho u (X0 = i kx' times it), rho v (X1), the shared
-  // form's D b_half (X2), and D w, added to X0: the thread reads back what it
-  // stored in the first run (from L2), which costs less than a second line of
-  // shared memory, hence half the CTAs.
-  constexpr int RUNS = MODE == ZFX_FIELDS ? 2 : MODE == ZFX_SHARED ? 4 : 3;
+  // A set's lines in turn: rho u (X0 = i kx' times it), then D w, added to X0: the
+  // thread reads back what it stored (from L2), which costs less than a second
+  // line of shared memory, hence half the blocks.
 #pragma unroll
-  for (int run = 0; run < RUNS; ++run) {
-    const bool wrun = MODE != ZFX_FIELDS && run >= 2;
-    const bool grad = MODE != ZFX_FIELDS && run == 0;        // times i kx'
-    const bool sum = MODE != ZFX_FIELDS && run == RUNS - 1;  // add to what X0 holds
-    cplx<T>* out = run == 1 ? X1 : (MODE == ZFX_SHARED && run == 2) ? X2 : X0;
-    if (MODE == ZFX_FIELDS && run == 1 && !v) return;  // one field
+  for (int run = 0; run < (MODE == ZFX_FIELDS ? 1 : 2); ++run) {
+    const bool sum = run == 1;
+    if (sum && set) return;
+    const bool grad = MODE != ZFX_FIELDS && set == 0 && !sum;  // times i kx'
+    cplx<T>* out = set == 0 ? X0 : set == 1 ? X1 : X2;
     if (run) __syncthreads();
-    if (wrun) z_first_fwd<T, C>(p, b0, RY, flux(sum ? w : bh, bh));
-    else z_first_fwd<T, C>(p, b0, RY, field(run ? v : u, MODE != ZFX_FIELDS));
+    if (MODE != ZFX_FIELDS && (sum || set == 2)) z_first_fwd<T, C>(p, b0, RY, flux(sum ? w : bh, bh));
+    else z_first_fwd<T, C>(p, b0, RY, field(set ? v : u, MODE != ZFX_FIELDS));
     __syncthreads();
 #pragma unroll 1
     for (int i = 1; i + 1 < p.np; ++i) {
@@ -599,10 +609,14 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
   }
 }
 
-// Inverse x transforms with the velocity correction.  Lines: i kx' phi~ (u),
-// psi~ (v), the level difference of phi~ (w; taken in the spectrum, so no halo
-// level is transformed and no difference of rounded potentials is formed) and,
-// where it is stored, phi~ itself.
+// Inverse x transforms with the velocity correction, a line per block: i kx' phi~
+// (u), psi~ (v) and
+//  * where the potential is not stored, the level difference of phi~ (w), taken in
+//    the spectrum: no halo level, no difference of rounded potentials;
+//  * where it is, phi~ itself, w corrected by the differences of the values
+//    stored (so a defect correction, which sees the state, also corrects their
+//    rounding).  Its blocks overlap by the level below their first interface:
+//    2 C levels, 2 C - 1 interfaces.
 template <class T, class TS, int MODE, int RL>
 __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
     const __grid_constant__ ZPlan p, GridK g, int RY, const cplx<T>* __restrict__ S1,
@@ -615,21 +629,28 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
   cplx<T>* b0 = reinterpret_cast<cplx<T>*>(smem_dyn);
   const int ny = g.ny, nz = g.nz;
   const int y0 = blockIdx.y * RY;
-  const int z = (blockIdx.x * C + (threadIdx.x & (C - 1))) * 2;
-  const bool on = z < nz, two = z + 1 < nz, vec = !(nz & 1);
+  // lines 0: d/dx (from S1), 1: d/dy (from S2), 2: d/dz or phi (from S1): the
+  // lines of a tile run side by side, so the tile's spectra still come from L2
+  const int runs = MODE == ZIX_FIELDS ? (S2 ? 2 : 1) : 3;
+  const int chunks = (nz + 2 * C - 1) / (2 * C);
+  int chunk = blockIdx.x / runs, run = blockIdx.x - chunk * runs;
+  if (MODE != ZIX_FIELDS && chunk >= chunks) {  // the potential's further blocks
+    chunk = blockIdx.x - 2 * chunks;
+    run = 2;
+  }
+  const bool pot = MODE != ZIX_FIELDS && MODE != ZIX_GRAD && run == 2 && phi_out;
+  const int c = threadIdx.x & (C - 1);
+  const int z = pot ? chunk * (2 * C - 1) - 1 + 2 * c : (chunk * C + c) * 2;
+  const bool on = z < nz, two = z + 1 < nz, one = z >= 0;
+  const bool vec = !(nz & 1) && !pot;
   const int rows = min(RY, ny - y0);
   const int xs = ny * nz, ws = ny * (nz + 1);
   const T idz = (T)(1.0 / g.dz);
   const T sd = (T)sdt;
 
-  // runs: d/dx (from S1), d/dy (from S2), d/dz (from S1), phi (from S1)
-  const int runs = MODE == ZIX_FIELDS ? (S2 ? 2 : 1) : (MODE != ZIX_GRAD && phi_out) ? 4 : 3;
-#pragma unroll 1
-  for (int run = 0; run < (MODE == ZIX_FIELDS ? 2 : MODE == ZIX_GRAD ? 3 : 4); ++run) {
-    if (run >= runs) break;
     const cplx<T>* src = run == 1 ? S2 : S1;
-    const bool gx = MODE != ZIX_FIELDS && run == 0, gz = MODE != ZIX_FIELDS && run == 2;
-    if (run) __syncthreads();
+    const bool gx = MODE != ZIX_FIELDS && run == 0;
+    const bool gz = MODE != ZIX_FIELDS && run == 2 && !pot;
     // First pass: wavenumbers t + Q j and their mirrors N - k of butterflies
     // t1 and t2, from the half spectra of the two levels.
     {
@@ -648,12 +669,12 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
         // loads in one batch: R / 2 wavenumbers of each butterfly
         cpair<T> x1[R / 2], x2[R / 2], xn;
 #pragma unroll
-        for (int j = 0; j < R / 2; ++j) x1[j] = ldcpair(q + (t1 + p.Q * j) * xs, vec, two);
+        for (int j = 0; j < R / 2; ++j) x1[j] = ldcpair(q + (t1 + p.Q * j) * xs, vec, two, one);
         if (has2) {
 #pragma unroll
-          for (int j = 0; j < R / 2; ++j) x2[j] = ldcpair(q + (t2 + p.Q * j) * xs, vec, two);
+          for (int j = 0; j < R / 2; ++j) x2[j] = ldcpair(q + (t2 + p.Q * j) * xs, vec, two, one);
         }
-        if (!s) xn = ldcpair(q + (p.N / 2) * xs, vec, two);
+        if (!s) xn = ldcpair(q + (p.N / 2) * xs, vec, two, one);
         if (gz) {
           // the difference to the level below (none at the surface)
           auto below = [&](int k, cpair<T>& x) {
@@ -709,26 +730,18 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
       z_mid_pass<T, C, true>(p, i, b0, RY, tw);
       __syncthreads();
     }
-    // Last pass.  Full-level fields: out = in - line, the line itself, or
-    // (the defect correction's potential) in + line.
-    if (!gz) {
-      const TS* in = run == 0 ? u_in : run == 1 ? v_in : phi_out;
-      TS* out = run == 0 ? u_out : run == 1 ? v_out : phi_out;
-      const bool plain = MODE == ZIX_FIELDS || MODE == ZIX_GRAD || (run == 3 && MODE != ZIX_REFINE);
-      const T sg = run == 3 ? (T)1 : (T)-1;
+    // Last pass.  The full-level lines: out = in - line, or the line itself.
+    if (run < 2) {
+      const TS* in = run == 0 ? u_in : v_in;
+      TS* out = run == 0 ? u_out : v_out;
       z_last_inv<T, C>(p, b0, RY, [&](auto rc, int row, int n, int step, const cplx<T>* q) {
         constexpr int R = decltype(rc)::value;
         if (!on || row >= rows) return;
         const int o = (n * ny + y0 + row) * nz + z;
         pair2<TS> a[R];
         if (MODE != ZIX_FIELDS && MODE != ZIX_GRAD) {
-          if (plain) {
 #pragma unroll
-            for (int j = 0; j < R; ++j) a[j].a = a[j].b = (TS)0;
-          } else {
-#pragma unroll
-            for (int j = 0; j < R; ++j) a[j] = ldpair(in + o + j * step * xs, vec, two);
-          }
+          for (int j = 0; j < R; ++j) a[j] = ldpair(in + o + j * step * xs, vec, two);
         }
         cplx<T> x[R];
 #pragma unroll
@@ -738,13 +751,70 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
         for (int j = 0; j < R; ++j) {
           TS r0 = (TS)x[j].x, r1 = (TS)x[j].y;
           if (MODE != ZIX_FIELDS && MODE != ZIX_GRAD) {
-            r0 = (TS)((T)a[j].a + sg * x[j].x);
-            r1 = (TS)((T)a[j].b + sg * x[j].y);
+            r0 = (TS)((T)a[j].a - x[j].x);
+            r1 = (TS)((T)a[j].b - x[j].y);
           }
           stpair(out + o + j * step * xs, r0, r1, vec, two);
         }
       });
-      continue;
+      return;
+    }
+    // The potential: levels z (but the block's first, the one below's) and z + 1
+    // are stored, and the interfaces at both get their difference.
+    if (pot) {
+      const unsigned group = (C == 32 ? ~0u : (1u << C) - 1) << ((threadIdx.x & 31) & ~(C - 1));
+      z_last_inv<T, C>(p, b0, RY, [&](auto rc, int row, int n, int step, const cplx<T>* q) {
+        constexpr int R = decltype(rc)::value;
+        if (row >= rows) return;  // the same for the lanes of a group
+        const int o = (n * ny + y0 + row) * nz + z, wo = (n * ny + y0 + row) * (nz + 1) + z;
+        const bool la = c > 0 && on, lb = two;
+        TS a[R], b[R], fa[R], fb[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+          a[j] = la ? w_in[wo + j * step * ws] : (TS)0;
+          b[j] = lb ? w_in[wo + j * step * ws + 1] : (TS)0;
+          if (MODE == ZIX_REFINE) {
+            fa[j] = la ? phi_out[o + j * step * xs] : (TS)0;
+            fb[j] = lb ? phi_out[o + j * step * xs + 1] : (TS)0;
+          }
+        }
+        if (MODE == ZIX_STAGE) {
+#pragma unroll
+          for (int j = 0; j < R; ++j) {
+            const TS* t = bh + wo + j * step * ws;
+            if (la) a[j] = (TS)zstage((T)a[j], sd, (T)t[0]);
+            if (lb) b[j] = (TS)zstage((T)b[j], sd, (T)t[1]);
+          }
+        }
+        cplx<T> x[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) x[j] = q[j * C];
+        zdft<T, R, true>(x);
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+          const T below = __shfl_up_sync(group, x[j].y, 1, C);
+          const int k = j * step * xs, kw = j * step * ws;
+          if (la) {
+            w_out[wo + kw] = (TS)((T)a[j] - (x[j].x - below) * idz);
+            phi_out[o + k] = (TS)(MODE == ZIX_REFINE ? (T)fa[j] + x[j].x : x[j].x);
+          }
+          if (lb) {  // no correction at the surface
+            const T d = one ? (x[j].y - x[j].x) * idz : (T)0;
+            w_out[wo + kw + 1] = (TS)((T)b[j] - d);
+            phi_out[o + k + 1] = (TS)(MODE == ZIX_REFINE ? (T)fb[j] + x[j].y : x[j].y);
+          }
+        }
+        // the lid level keeps the input's value (stages: with its buoyancy)
+        if ((MODE == ZIX_STAGE || w_out != w_in) && ((la && z == nz - 1) || (lb && z + 2 == nz))) {
+          for (int j = 0; j < R; ++j) {
+            const int top = wo + j * step * ws + (nz - z);
+            TS t = w_in[top];
+            if (MODE == ZIX_STAGE) t = (TS)zstage((T)t, sd, (T)bh[top]);
+            w_out[top] = t;
+          }
+        }
+      });
+      return;
     }
     z_last_inv<T, C>(p, b0, RY, [&](auto rc, int row, int n, int step, const cplx<T>* line) {
       constexpr int R = decltype(rc)::value;
@@ -792,7 +862,6 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
         }
       }
     });
-  }
 }
 
 // ---- y lines ---------------------------------------------------------------------

@@ -72,4 +72,21 @@ template <class T>
 cudaError_t ziy(bool grad, const ZLine<T>& l, const GridK& g, const cplx<T>* in, double scale,
                 cplx<T>* out0, cplx<T>* out1, cudaStream_t st);
 
+// One kx plane per block (zplane.cuh): forward y, the vertical solve, inverse y.
+// X1 null: the source is F(X0) alone; fwd false: X0 is the source's spectrum.
+// out1 = F^-1(i ky' phi^), null: out0 = phi~ alone.
+struct ZSolve {
+  const double* inv;          // reciprocal pivots (nx / 2 + 1, nz, ny)
+  cplx<double>* dpd;          // scratch of that shape, single precision only
+  const unsigned char* lw;    // per 32 columns: long waves (single precision)
+};
+// level chunks per group of the plane's scratch; 0: the plane does not fit
+template <class T>
+int zplane_group(const ZPlan& p, int nz);
+template <class T>
+cudaError_t zplane(const ZLine<T>& l, const GridK& g, const ThomasK& t, const ZSolve& s,
+                   bool fwd, const cplx<T>* X0, const cplx<T>* X1, cplx<T>* out0, cplx<T>* out1,
+                   cudaStream_t st);
+cudaError_t zplane_inv(const GridK& g, const ThomasK& t, double* inv, cudaStream_t st);
+
 }  // namespace ob

@@ -16,7 +16,7 @@ from tests.gpu_helpers import dev, host
 
 pytestmark = pytest.mark.gpu
 
-GRIDS = [(8, 10, 3), (16, 12, 9), (50, 36, 17), (162, 40, 8), (36, 162, 33), (250, 8, 5),
+GRIDS = [(8, 10, 9), (16, 12, 9), (50, 36, 17), (162, 40, 8), (36, 162, 33), (250, 8, 5),
          (128, 96, 16), (972, 8, 4), (8, 1000, 7), (1024, 16, 17)]
 
 
@@ -45,8 +45,12 @@ def _close(got, want, bar, what):
 
 @pytest.mark.parametrize("nx, ny, nz", GRIDS)
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
-def test_projection_and_operators_match_the_oracle(nx, ny, nz, prec):
+@pytest.mark.parametrize("plane", [1, 0])
+def test_projection_and_operators_match_the_oracle(nx, ny, nz, prec, plane):
     p, rho0 = _plan(nx, ny, nz, prec, damping=True, epsilon=0.5)
+    if plane and not p.variants()["z_yz"]:
+        pytest.skip("the plane does not fit shared memory")
+    p.set_variants(z_yz=plane)
     dt = p.dtype
     u, v, w = _fields(nx, ny, nz, seed=nx + 7 * ny + nz)
     wind, fine, rough = (1e-12,) * 3 if prec == "fp64" else (1e-6, 1e-5, 1e-3)
