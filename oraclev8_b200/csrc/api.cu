@@ -252,6 +252,7 @@ struct OraclePlan {
   int refine_passes = 0, refine_every = 1;
   long step_count = 0;
   int capturing = 0;  // recording a step graph: no solver-residual logging
+  unsigned logged = 0;  // diag slots that hold a logged solve's residuals
   size_t esz = 8;  // element size of T
   // device constants
   double *kx = nullptr, *ky = nullptr, *rho = nullptr, *rhoh = nullptr, *theta0 = nullptr;
@@ -282,7 +283,7 @@ struct OraclePlan {
   unsigned char* lw_flag = nullptr;
   int n_lw = 0;
   float* tcoef = nullptr;  // FP32 plans: (negs, rho, a, c) per level, as float4
-  float* gth = nullptr;    // FP32 plans: g / theta0 per level
+  void* gth = nullptr;     // g / theta0 per level, in the plan's type
   cudaStream_t aux = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // launch accounting and optional per-kernel-class event timing
@@ -1341,12 +1342,24 @@ int project_impl(OraclePlan* p, const T* u, const T* v, const T* w, const T* th,
   const int de = p->diag_every < 1 ? 1 : p->diag_every;
   const bool log = !p->capturing && ((de == 1) || (p->solve_count % de == 1));
   double* diag = nullptr;
+  // The residual slots of a solve that does not log read zero.  They are zero
+  // until one logs, so only its traces are cleared: at once in recorded work,
+  // which may run after one that logged (a step clears all its own in one go),
+  // and else where one did.  Two clears a projection took 15 us of a step's 400
+  // at 96 x 96 x 32.
+  const unsigned bits = (1u << slot_c) | (1u << slot_d);
   if (log) {
     diag = p->diag;
     OB_CUDA(cudaMemsetAsync(p->diag + slot_d, 0, sizeof(double), st));
-  } else {
-    OB_CUDA(cudaMemsetAsync(p->diag + slot_c, 0, sizeof(double), st));
-    OB_CUDA(cudaMemsetAsync(p->diag + slot_d, 0, sizeof(double), st));
+    p->logged |= bits;
+  } else if (!p->capturing) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    OB_CUDA(cudaStreamIsCapturing(st, &cap));
+    if ((p->logged & bits) || cap != cudaStreamCaptureStatusNone) {
+      OB_CUDA(cudaMemsetAsync(p->diag + slot_c, 0, sizeof(double), st));
+      OB_CUDA(cudaMemsetAsync(p->diag + slot_d, 0, sizeof(double), st));
+    }
+    if (cap == cudaStreamCaptureStatusNone) p->logged &= ~bits;
   }
   const bool stage = stage_sdt >= 0.0;
   if (shared && sizeof(T) == 4 && stage) {
@@ -1592,8 +1605,7 @@ SlowK slow_args(const OraclePlan* p) {
   s.sponge = p->sponge;
   s.diff = p->diffusion;
   s.cool = p->cooling;
-  s.drag_cd = p->drag_cd;
-  s.drag_dz = p->drag_dz;
+  s.drag_rate = p->drag_cd / p->drag_dz;
   s.drag_u_env = p->drag_u_env;
   s.drag_v_env = p->drag_v_env;
   s.drag_w = p->drag_w;
@@ -1602,8 +1614,8 @@ SlowK slow_args(const OraclePlan* p) {
   s.sp_a = p->sp_a;
   s.sp_ah = p->sp_ah;
   s.diff_nu = p->diff_nu;
-  s.diff_dx2 = p->diff_dx2;
-  s.diff_dy2 = p->diff_dy2;
+  s.diff_rdx2 = 1.0 / p->diff_dx2;
+  s.diff_rdy2 = 1.0 / p->diff_dy2;
   s.lap_u = p->Lu;
   s.lap_v = p->Lv;
   s.cool_alpha = p->cool_alpha;
@@ -1726,7 +1738,7 @@ int slow_impl(OraclePlan* p, int mask, double dts, const T* u, const T* v, const
   if ((mask & OB_TEND_DIFFUSION) && p->diffusion == OB_DIFF_BIHARMONIC) {
     const dim3 lg((unsigned)((p->g.ny * p->g.nz + 255) / 256), (unsigned)p->g.nx);
     { Launch L_(p, 5, st); k_lap2<T><<<lg, 256, 0, st>>>(
-          p->g, u, v, p->diff_dx2, p->diff_dy2, (T*)p->Lu, (T*)p->Lv); }
+          p->g, u, v, 1.0 / p->diff_dx2, 1.0 / p->diff_dy2, (T*)p->Lu, (T*)p->Lv); }
     OB_LAUNCHED();
   }
   // production components run in the gather kernels
@@ -1766,10 +1778,14 @@ int copy_field(void* dst, const void* src, size_t n, cudaStream_t st) {
 template <class T>
 int diag_impl(OraclePlan* p, const T* u, const T* v, const T* w, const T* th, const T* phi,
               cudaStream_t st) {
-  { Launch L_(p, 6, st); k_diag_partial<T><<<p->nparts, 256, 0, st>>>(p->g, u, v, w, th, phi, p->parts); }
+  // 8 vectors a thread and field, up to four blocks per SM
+  const long n = (long)p->g.nx * p->g.ny * p->g.nz;
+  const int nb = (int)std::min<long>(p->nparts, n * (long)sizeof(T) / (16 * 8 * kDiagThreads) + 1);
+  { Launch L_(p, 6, st); k_diag_partial<T><<<nb, kDiagThreads, 0, st>>>(p->g, u, v, w, th, phi,
+                                                                       p->parts); }
   OB_LAUNCHED();
-  { Launch L_(p, 6, st); k_diag_final<<<1, 32, 0, st>>>(p->parts, p->nparts,
-                                 (double)p->g.nx * p->g.ny * p->g.nz, p->blowup_u, p->diag); }
+  { Launch L_(p, 6, st); k_diag_final<<<1, kDiagThreads, 0, st>>>(p->parts, nb, (double)n,
+                                                                 p->blowup_u, p->diag); }
   OB_LAUNCHED();
   return OB_OK;
 }
@@ -1787,6 +1803,9 @@ int step_impl(OraclePlan* p, const OracleStatePtrs* in, const OracleStatePtrs* o
                    p->diffusion;
   const int all = OB_TEND_ADVECTION | OB_TEND_CORIOLIS | OB_TEND_DAMPING | OB_TEND_HEATING |
                   OB_TEND_DRAG | OB_TEND_SPONGE | OB_TEND_DIFFUSION | OB_TEND_COOLING;
+  if (p->capturing)
+    OB_CUDA(cudaMemsetAsync(p->diag + OB_DIAG_COMPAT0, 0,
+                            (OB_DIAG_LAST_DISC + 1 - OB_DIAG_COMPAT0) * sizeof(double), st));
   // anchor state y^n after the first slow half step
   const T *au = (const T*)in->u, *av = (const T*)in->v, *aw = (const T*)in->w,
           *ath = (const T*)in->theta_prime, *aphi = (const T*)in->phi;
@@ -1821,7 +1840,7 @@ int step_impl(OraclePlan* p, const OracleStatePtrs* in, const OracleStatePtrs* o
     if (p->Bh) {
       const long ncol = (long)p->g.nx * p->g.ny;
       { Launch L_(p, 7, st); k_bhalf<T><<<(unsigned)std::min<long>((ncol + 7) / 8, 65535), 256, 0, st>>>(
-          p->g, ath, p->theta0, p->gth, (T*)p->Bh); }
+          p->g, ath, (const T*)p->gth, (T*)p->Bh); }
       OB_LAUNCHED();
       bh = (const T*)p->Bh;
     }
@@ -3114,14 +3133,15 @@ int oracle_b200_plan_create(const OracleGridDesc* grid, const OracleComponentDes
     if ((rc = dalloc(p, &p->tcoef, coef.size() * sizeof(float)))) return bail(rc);
     OB_CUDA(cudaMemcpyAsync(p->tcoef, coef.data(), coef.size() * sizeof(float),
                             cudaMemcpyHostToDevice, p->astream));
-    std::vector<float> gth(nz);
-    for (int k = 0; k < nz; ++k) gth[k] = (float)(kGravity / comp->theta0[k]);
-    if ((rc = dalloc(p, &p->gth, gth.size() * sizeof(float)))) return bail(rc);
-    OB_CUDA(cudaMemcpyAsync(p->gth, gth.data(), gth.size() * sizeof(float),
-                            cudaMemcpyHostToDevice, p->astream));
     // the vectors must outlive the copies: pageable copies are staged before
     // the call returns
   }
+  std::vector<double> gthd(nz);
+  for (int k = 0; k < nz; ++k) gthd[k] = kGravity / comp->theta0[k];
+  const std::vector<float> gthf(gthd.begin(), gthd.end());
+  if ((rc = dalloc(p, &p->gth, nz * e))) return bail(rc);
+  OB_CUDA(cudaMemcpyAsync(p->gth, p->prec == OB_PREC_F64 ? (const void*)gthd.data() : gthf.data(),
+                          nz * e, cudaMemcpyHostToDevice, p->astream));
   if ((rc = dalloc(p, &p->diag, 64 * sizeof(double)))) return bail(rc);
   // ordered after the allocation on the set-up stream
   OB_CUDA(cudaMemsetAsync(p->diag, 0, 64 * sizeof(double), p->astream));

@@ -863,12 +863,12 @@ struct SlowK {
   double inv2dx, inv2dy, inv60dx, inv60dy, inv2dz, invdz;
   // production components, in slot order after Coriolis (operator_config.py:147-160)
   int drag, sponge, diff, cool;
-  double drag_cd, drag_dz, drag_u_env, drag_v_env;
+  double drag_rate, drag_u_env, drag_v_env;  // drag_rate: Cd / dz
   const double* drag_w;  // (nz) max(0, 1 - z / H_bl)
   double sp_u_env, sp_v_env;
   const double* sp_a;    // (nz) full levels
   const double* sp_ah;   // (nz+1) half levels
-  double diff_nu, diff_dx2, diff_dy2;
+  double diff_nu, diff_rdx2, diff_rdy2;  // reciprocals of dx^2, dy^2
   const void* lap_u;     // biharmonic: lap(u), lap(v) of this slow half (element type T)
   const void* lap_v;
   double cool_alpha;
@@ -879,23 +879,16 @@ constexpr int kTendDrag = 16, kTendSponge = 32, kTendDiffusion = 64, kTendCoolin
 
 // Periodic 5-point horizontal Laplacian of q at o, in the reference's order
 // ((q[i+1] - 2 q) + q[i-1]) / dx2 + ((q[j+1] - 2 q) + q[j-1]) / dy2
-// (tendency.py:1551-1558, 1608-1613).  off[2], off[3]: offsets of i-1, i+1.
+// (tendency.py:1551-1558, 1608-1613), by the spacings' reciprocals: the two
+// divisions per Laplacian were most of the double-precision kernels' arithmetic
+// (320 x 320 x 32, production: a slow half with its inner Laplacian 259 us).
+// off[2], off[3]: offsets of i-1, i+1.
 template <class T, class A>
 __device__ __forceinline__ A lap5(const T* __restrict__ q, int o, const int* offx,
-                                  const int* offy, A dx2, A dy2) {
+                                  const int* offy, A rdx2, A rdy2) {
   const A c = (A)q[o];
-  return ((A)q[o + offx[3]] - (A)2 * c + (A)q[o + offx[2]]) / dx2 +
-         ((A)q[o + offy[3]] - (A)2 * c + (A)q[o + offy[2]]) / dy2;
-}
-
-// The same Laplacian with the spacings' reciprocals, for single-precision
-// state: two multiplies where lap5 takes two IEEE divisions (the FP32 path is
-// held to its rounding, not to the reference's operation order).
-__device__ __forceinline__ float lap5r(const float* __restrict__ q, int o, const int* offx,
-                                       const int* offy, float rdx2, float rdy2) {
-  const float c = q[o];
-  return (q[o + offx[3]] - 2.0f * c + q[o + offx[2]]) * rdx2 +
-         (q[o + offy[3]] - 2.0f * c + q[o + offy[2]]) * rdy2;
+  return ((A)q[o + offx[3]] - (A)2 * c + (A)q[o + offx[2]]) * rdx2 +
+         ((A)q[o + offy[3]] - (A)2 * c + (A)q[o + offy[2]]) * rdy2;
 }
 
 // WS5 upwind derivative along one horizontal axis.  cols[r] are the linear
@@ -971,6 +964,12 @@ __global__ void __launch_bounds__(256) k_slow(GridK g, SlowK s, int mask, double
     offyw[r] = (jy[r] - j) * nzw;
   }
   const bool ws5 = (s.adv == 2);
+  double dragc = 0.0;  // the column's surface drag rate
+  if (drg) {
+    const double up0 = (double)u[col * nz] - s.drag_u_env;
+    const double vp0 = (double)v[col * nz] - s.drag_v_env;
+    dragc = s.drag_rate * sqrt(up0 * up0 + vp0 * vp0);
+  }
   for (int k = threadIdx.x; k <= nz; k += blockDim.x) {
     const int o = col * nz + k;
     const int ow = col * nzw + k;
@@ -1019,9 +1018,7 @@ __global__ void __launch_bounds__(256) k_slow(GridK g, SlowK s, int mask, double
         tv = tv + (-f) * (uc - s.u_env);
       }
       if (drg) {  // SurfaceDragComponent (tendency.py:1318-1338)
-        const double up0 = (double)u[col * nz] - s.drag_u_env;
-        const double vp0 = (double)v[col * nz] - s.drag_v_env;
-        const double al = s.drag_cd * sqrt(up0 * up0 + vp0 * vp0) / s.drag_dz * s.drag_w[k];
+        const double al = dragc * s.drag_w[k];
         tu = tu + (-al) * (uc - s.drag_u_env);
         tv = tv + (-al) * (vc - s.drag_v_env);
       }
@@ -1032,13 +1029,13 @@ __global__ void __launch_bounds__(256) k_slow(GridK g, SlowK s, int mask, double
         tt = tt + (-a) * thc;
       }
       if (dif == 1) {  // HorizontalDiffusionComponent (tendency.py:1548-1562)
-        tu = tu + s.diff_nu * lap5<T, double>(u, o, offx, offy, s.diff_dx2, s.diff_dy2);
-        tv = tv + s.diff_nu * lap5<T, double>(v, o, offx, offy, s.diff_dx2, s.diff_dy2);
+        tu = tu + s.diff_nu * lap5<T, double>(u, o, offx, offy, s.diff_rdx2, s.diff_rdy2);
+        tv = tv + s.diff_nu * lap5<T, double>(v, o, offx, offy, s.diff_rdx2, s.diff_rdy2);
       } else if (dif == 2) {  // HyperDiffusionComponent (tendency.py:1615-1621)
         const T* lu = static_cast<const T*>(s.lap_u);
         const T* lv = static_cast<const T*>(s.lap_v);
-        tu = tu + (-s.diff_nu) * lap5<T, double>(lu, o, offx, offy, s.diff_dx2, s.diff_dy2);
-        tv = tv + (-s.diff_nu) * lap5<T, double>(lv, o, offx, offy, s.diff_dx2, s.diff_dy2);
+        tu = tu + (-s.diff_nu) * lap5<T, double>(lu, o, offx, offy, s.diff_rdx2, s.diff_rdy2);
+        tv = tv + (-s.diff_nu) * lap5<T, double>(lv, o, offx, offy, s.diff_rdx2, s.diff_rdy2);
       }
       if (col_) tt = tt + (-s.cool_alpha) * thc;  // NewtonianCooling (tendency.py:1661-1662)
       if (dmp) {
@@ -1133,8 +1130,8 @@ __global__ void __launch_bounds__(256, PROD ? 5 : 4) k_slow_f32(GridK g, SlowK s
   const bool spg = PROD && (mask & kTendSponge) && s.sponge;
   const int dif = (PROD && (mask & kTendDiffusion)) ? s.diff : 0;
   const bool col_ = PROD && (mask & kTendCooling) && s.cool;
-  const float dnu = (float)s.diff_nu, rdx2 = (float)(1.0 / s.diff_dx2),
-              rdy2 = (float)(1.0 / s.diff_dy2);
+  const float dnu = (float)s.diff_nu, rdx2 = (float)s.diff_rdx2,
+              rdy2 = (float)s.diff_rdy2;
   int offx[6], offy[6], offxw[6], offyw[6];
   const int dd[6] = {-3, -2, -1, 1, 2, 3};
 #pragma unroll
@@ -1202,7 +1199,7 @@ __global__ void __launch_bounds__(256, PROD ? 5 : 4) k_slow_f32(GridK g, SlowK s
       if (drg) {
         const float du_env = (float)s.drag_u_env, dv_env = (float)s.drag_v_env;
         const float up0 = u[col * nz] - du_env, vp0 = v[col * nz] - dv_env;
-        const float al = (float)s.drag_cd * sqrtf(up0 * up0 + vp0 * vp0) / (float)s.drag_dz *
+        const float al = (float)s.drag_rate * sqrtf(up0 * up0 + vp0 * vp0) *
                          (float)s.drag_w[k];
         tu = tu + (-al) * (uc - du_env);
         tv = tv + (-al) * (vc - dv_env);
@@ -1214,13 +1211,13 @@ __global__ void __launch_bounds__(256, PROD ? 5 : 4) k_slow_f32(GridK g, SlowK s
         tt = tt + (-a) * thc;
       }
       if (dif == 1) {
-        tu = tu + dnu * lap5r(u, o, offx, offy, rdx2, rdy2);
-        tv = tv + dnu * lap5r(v, o, offx, offy, rdx2, rdy2);
+        tu = tu + dnu * lap5<float, float>(u, o, offx, offy, rdx2, rdy2);
+        tv = tv + dnu * lap5<float, float>(v, o, offx, offy, rdx2, rdy2);
       } else if (dif == 2) {
         const float* lu = static_cast<const float*>(s.lap_u);
         const float* lv = static_cast<const float*>(s.lap_v);
-        tu = tu + (-dnu) * lap5r(lu, o, offx, offy, rdx2, rdy2);
-        tv = tv + (-dnu) * lap5r(lv, o, offx, offy, rdx2, rdy2);
+        tu = tu + (-dnu) * lap5<float, float>(lu, o, offx, offy, rdx2, rdy2);
+        tv = tv + (-dnu) * lap5<float, float>(lv, o, offx, offy, rdx2, rdy2);
       }
       if (col_) tt = tt + (-(float)s.cool_alpha) * thc;
       if (dmp) {
@@ -1521,7 +1518,7 @@ __global__ void __launch_bounds__(256, 3) k_slow_xw(GridK g, SlowK s, int mask, 
 // only division is r / nz (32-bit: nx ny (nz + 1) < 2^31, plan_create).
 template <class T>
 __global__ void __launch_bounds__(256) k_lap2(GridK g, const T* __restrict__ u,
-                                              const T* __restrict__ v, double dx2, double dy2,
+                                              const T* __restrict__ v, double rdx2, double rdy2,
                                               T* __restrict__ lu, T* __restrict__ lv) {
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int pl = ny * nz;
@@ -1535,14 +1532,8 @@ __global__ void __launch_bounds__(256) k_lap2(GridK g, const T* __restrict__ u,
     const int o = i * pl + r;
     const int offx[6] = {0, 0, (im - i) * pl, (ip - i) * pl, 0, 0};
     const int offy[6] = {0, 0, (jm - j) * nz, (jp - j) * nz, 0, 0};
-    if (sizeof(T) == 8) {
-      lu[o] = (T)lap5<T, double>(u, o, offx, offy, dx2, dy2);
-      lv[o] = (T)lap5<T, double>(v, o, offx, offy, dx2, dy2);
-    } else {
-      const float rdx2 = (float)(1.0 / dx2), rdy2 = (float)(1.0 / dy2);
-      lu[o] = (T)lap5r((const float*)u, o, offx, offy, rdx2, rdy2);
-      lv[o] = (T)lap5r((const float*)v, o, offx, offy, rdx2, rdy2);
-    }
+    lu[o] = lap5<T, T>(u, o, offx, offy, (T)rdx2, (T)rdy2);
+    lv[o] = lap5<T, T>(v, o, offx, offy, (T)rdx2, (T)rdy2);
   }
 }
 
@@ -1631,158 +1622,127 @@ __global__ void k_neg_ksq(GridK g, const cplx<T>* __restrict__ in, const double*
 
 // ---------------------------------------------------------------------------
 // Step diagnostics (integrator.py:287-295): max|u|, max|v|, max|w|, max|th|,
-// sum(phi), min/max phi[:, :, 0].  Two-stage deterministic reduction.
+// sum(phi), min/max phi[:, :, 0].  Two-stage deterministic reduction: a block's
+// partials, combined in their order by one block.  Bound by memory at large grids
+// (16-byte loads; 512 x 512 x 64 double, 671 MB: 173 us with one value a load),
+// by latency at small ones, which get no more blocks than their loads fill (one
+// warp over 592 partials took longer than the sums).
 // ---------------------------------------------------------------------------
 struct DiagPart {
-  double mu, mv, mw, mt, sp, pmin, pmax, pad;
+  double v[8];  // max|u|, max|v|, max|w|, max|th|, sum phi, min, max phi_0, unused
 };
 
 // Maximum and minimum that propagate NaN as NumPy's max / min do (fmax and
 // fmin would drop it): once either operand is NaN the result stays NaN.
-__device__ __forceinline__ double nan_max(double m, double x) { return (x > m || x != x) ? x : m; }
-__device__ __forceinline__ double nan_min(double m, double x) { return (x < m || x != x) ? x : m; }
-__device__ __forceinline__ float nan_maxf(float m, float x) { return (x > m || x != x) ? x : m; }
-
 template <class T>
-__global__ void __launch_bounds__(256) k_diag_partial(GridK g, const T* __restrict__ u,
-                                                      const T* __restrict__ v,
-                                                      const T* __restrict__ w,
-                                                      const T* __restrict__ th,
-                                                      const T* __restrict__ phi, DiagPart* part) {
-  const size_t n = (size_t)g.nx * g.ny * g.nz;
-  const size_t nw = (size_t)g.nx * g.ny * (g.nz + 1);
-  double mu = 0, mv = 0, mw = 0, mt = 0, sp = 0, pmin = INFINITY, pmax = -INFINITY;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  const size_t first = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  bool done = false;
-  if constexpr (sizeof(T) == 4) {
-    // single precision: float4 loads where sizes and pointers allow; the
-    // maxima of |.| are exact in float, the phi sum stays in double
-    const size_t al = reinterpret_cast<size_t>(u) | reinterpret_cast<size_t>(v) |
-                      reinterpret_cast<size_t>(w) | reinterpret_cast<size_t>(th) |
-                      reinterpret_cast<size_t>(phi);
-    if ((n & 3) == 0 && (nw & 3) == 0 && (al & 15) == 0) {
-      float fu = 0.0f, fv = 0.0f, fw = 0.0f, ft = 0.0f;
-      const float4* u4 = reinterpret_cast<const float4*>(u);
-      const float4* v4 = reinterpret_cast<const float4*>(v);
-      const float4* t4 = reinterpret_cast<const float4*>(th);
-      const float4* p4 = reinterpret_cast<const float4*>(phi);
-      const float4* w4 = reinterpret_cast<const float4*>(w);
-      auto amax = [](float m, float4 a) {
-        return nan_maxf(nan_maxf(nan_maxf(m, fabsf(a.x)), nan_maxf(fabsf(a.y), fabsf(a.z))),
-                        fabsf(a.w));
-      };
-      for (size_t e = first; e < n / 4; e += stride) {
-        const float4 a = u4[e], b = v4[e], c = t4[e], d = p4[e];
-        fu = amax(fu, a);
-        fv = amax(fv, b);
-        ft = amax(ft, c);
-        sp += (double)d.x;
-        sp += (double)d.y;
-        sp += (double)d.z;
-        sp += (double)d.w;
-      }
-      for (size_t e = first; e < nw / 4; e += stride) fw = amax(fw, w4[e]);
-      mu = fu;
-      mv = fv;
-      mw = fw;
-      mt = ft;
-      done = true;
-    }
-  }
-  if (!done) {
-    for (size_t e = first; e < n; e += stride) {
-      mu = nan_max(mu, fabs((double)u[e]));
-      mv = nan_max(mv, fabs((double)v[e]));
-      mt = nan_max(mt, fabs((double)th[e]));
-      sp += (double)phi[e];
-    }
-    for (size_t e = first; e < nw; e += stride) mw = nan_max(mw, fabs((double)w[e]));
-  }
-  // surface level k = 0 of every column
-  const size_t ncol = (size_t)g.nx * g.ny;
-  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < ncol; c += stride) {
-    const double p = phi[c * g.nz];
-    pmin = nan_min(pmin, p);
-    pmax = nan_max(pmax, p);
-  }
-  __shared__ double red[8][8];
-  double vals[7] = {mu, mv, mw, mt, sp, pmin, pmax};
+__device__ __forceinline__ T nan_max(T m, T x) { return (x > m || x != x) ? x : m; }
+template <class T>
+__device__ __forceinline__ T nan_min(T m, T x) { return (x < m || x != x) ? x : m; }
+__device__ __forceinline__ double diag_op(int q, double x, double y) {
+  return q == 4 ? x + y : q == 5 ? nan_min(x, y) : nan_max(x, y);
+}
+
+constexpr int kDiagThreads = 256;
+
+// Combines vals over the block in a fixed order; the result in thread 0.
+__device__ __forceinline__ void diag_block(double* vals, double (*red)[8]) {
 #pragma unroll
   for (int q = 0; q < 7; ++q) {
     double x = vals[q];
-    for (int o = 16; o > 0; o >>= 1) {
-      const double y = __shfl_xor_sync(0xffffffffu, x, o);
-      x = (q == 4) ? x + y : (q == 5 ? nan_min(x, y) : nan_max(x, y));
-    }
+    for (int o = 16; o > 0; o >>= 1) x = diag_op(q, x, __shfl_xor_sync(0xffffffffu, x, o));
     vals[q] = x;
   }
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0)
-    for (int q = 0; q < 7; ++q) red[wid][q] = vals[q];
+  __syncthreads();  // red may hold an earlier result
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int q = 0; q < 7; ++q) red[threadIdx.x >> 5][q] = vals[q];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw_ = blockDim.x >> 5;
-    double r[7];
-    for (int q = 0; q < 7; ++q) r[q] = red[0][q];
-    for (int ww = 1; ww < nw_; ++ww)
-      for (int q = 0; q < 7; ++q)
-        r[q] = (q == 4) ? r[q] + red[ww][q]
-                        : (q == 5 ? nan_min(r[q], red[ww][q]) : nan_max(r[q], red[ww][q]));
-    DiagPart p;
-    p.mu = r[0];
-    p.mv = r[1];
-    p.mw = r[2];
-    p.mt = r[3];
-    p.sp = r[4];
-    p.pmin = r[5];
-    p.pmax = r[6];
-    p.pad = 0;
-    part[blockIdx.x] = p;
-  }
+  if (threadIdx.x == 0)
+    for (int w = 1; w < kDiagThreads / 32; ++w)
+#pragma unroll
+      for (int q = 0; q < 7; ++q) vals[q] = diag_op(q, vals[q], red[w][q]);
 }
 
-// One warp combines the per-CTA partials (fixed order: lane-strided, then a
-// butterfly), so the result does not depend on timing.  It also raises the
-// plan's sticky blow-up flag diag[14] (OB_DIAG_BLOWUP): 1 for a non-finite
-// value in any field, 2 for max|u| above umax_limit (> 0), the blow-up test
-// of the reference's harness (measure_lh82_phase3.py:129-130).
-__global__ void k_diag_final(const DiagPart* part, int np, double ncell, double umax_limit,
-                             double* diag) {
-  if (blockIdx.x != 0 || threadIdx.x >= 32) return;
-  double mu = 0, mv = 0, mw = 0, mt = 0, sp = 0, pmin = INFINITY, pmax = -INFINITY;
-  for (int b = threadIdx.x; b < np; b += 32) {
-    const DiagPart q = part[b];
-    mu = nan_max(mu, q.mu);
-    mv = nan_max(mv, q.mv);
-    mw = nan_max(mw, q.mw);
-    mt = nan_max(mt, q.mt);
-    sp += q.sp;
-    pmin = nan_min(pmin, q.pmin);
-    pmax = nan_max(pmax, q.pmax);
+template <class T>
+__global__ void __launch_bounds__(kDiagThreads) k_diag_partial(
+    GridK g, const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ w,
+    const T* __restrict__ th, const T* __restrict__ phi, DiagPart* part) {
+  constexpr int V = 16 / sizeof(T);
+  struct __align__(16) Vec { T a[V]; };
+  const int n = g.nx * g.ny * g.nz, nw = g.nx * g.ny * (g.nz + 1);
+  // the maxima of |.| are exact in the fields' type, the phi sum in double
+  T m[4] = {(T)0, (T)0, (T)0, (T)0};
+  double sp = 0, pmin = INFINITY, pmax = -INFINITY;
+  const int stride = gridDim.x * kDiagThreads, first = blockIdx.x * kDiagThreads + threadIdx.x;
+  const size_t al = reinterpret_cast<size_t>(u) | reinterpret_cast<size_t>(v) |
+                    reinterpret_cast<size_t>(w) | reinterpret_cast<size_t>(th) |
+                    reinterpret_cast<size_t>(phi);
+  const int nv = (al & 15) == 0 ? n / V : 0, nwv = (al & 15) == 0 ? nw / V : 0;
+  auto vec = [](const T* p, int e) { return reinterpret_cast<const Vec*>(p)[e]; };
+  auto amax = [](T x, const Vec& a) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) x = nan_max(x, a.a[i] < (T)0 ? -a.a[i] : a.a[i]);
+    return x;
+  };
+#pragma unroll 2
+  for (int e = first; e < nv; e += stride) {
+    const Vec a = vec(u, e), b = vec(v, e), c = vec(th, e), d = vec(phi, e);
+    m[0] = amax(m[0], a);
+    m[1] = amax(m[1], b);
+    m[3] = amax(m[3], c);
+#pragma unroll
+    for (int i = 0; i < V; ++i) sp += (double)d.a[i];
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    mu = nan_max(mu, __shfl_xor_sync(0xffffffffu, mu, o));
-    mv = nan_max(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-    mw = nan_max(mw, __shfl_xor_sync(0xffffffffu, mw, o));
-    mt = nan_max(mt, __shfl_xor_sync(0xffffffffu, mt, o));
-    sp += __shfl_xor_sync(0xffffffffu, sp, o);
-    pmin = nan_min(pmin, __shfl_xor_sync(0xffffffffu, pmin, o));
-    pmax = nan_max(pmax, __shfl_xor_sync(0xffffffffu, pmax, o));
+#pragma unroll 4
+  for (int e = first; e < nwv; e += stride) m[2] = amax(m[2], vec(w, e));
+  // what the vectors leave
+  auto abs1 = [](T x) { return x < (T)0 ? -x : x; };
+  for (int e = nv * V + first; e < n; e += stride) {
+    m[0] = nan_max(m[0], abs1(u[e]));
+    m[1] = nan_max(m[1], abs1(v[e]));
+    m[3] = nan_max(m[3], abs1(th[e]));
+    sp += (double)phi[e];
   }
+  for (int e = nwv * V + first; e < nw; e += stride) m[2] = nan_max(m[2], abs1(w[e]));
+  // surface level k = 0 of every column
+  for (int c = first; c < g.nx * g.ny; c += stride) {
+    const double p = phi[(size_t)c * g.nz];
+    pmin = nan_min(pmin, p);
+    pmax = nan_max(pmax, p);
+  }
+  __shared__ double red[kDiagThreads / 32][8];
+  double vals[7] = {(double)m[0], (double)m[1], (double)m[2], (double)m[3], sp, pmin, pmax};
+  diag_block(vals, red);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int q = 0; q < 7; ++q) part[blockIdx.x].v[q] = vals[q];
+}
+
+// Combines the np blocks' partials and raises the plan's sticky blow-up flag
+// diag[14] (OB_DIAG_BLOWUP): 1 for a non-finite value in any field, 2 for max|u|
+// above umax_limit (> 0), the blow-up test of the reference's harness
+// (measure_lh82_phase3.py:129-130).  One block.
+__global__ void __launch_bounds__(kDiagThreads) k_diag_final(const DiagPart* part, int np,
+                                                             double ncell, double umax_limit,
+                                                             double* diag) {
+  __shared__ double red[kDiagThreads / 32][8];
+  double vals[7] = {0.0, 0.0, 0.0, 0.0, 0.0, INFINITY, -INFINITY};
+  for (int b = threadIdx.x; b < np; b += kDiagThreads)
+#pragma unroll
+    for (int q = 0; q < 7; ++q) vals[q] = diag_op(q, vals[q], part[b].v[q]);
+  diag_block(vals, red);
   if (threadIdx.x != 0) return;
-  const double mean = sp / ncell;
-  diag[0] = mu;
-  diag[1] = mv;
-  diag[2] = mw;
-  diag[3] = mt;
-  diag[4] = pmin - mean;
-  diag[5] = pmax - mean;
-  const bool finite = isfinite(mu) && isfinite(mv) && isfinite(mw) && isfinite(mt) &&
-                      isfinite(sp) && isfinite(pmin) && isfinite(pmax);
+  const double mean = vals[4] / ncell;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) diag[q] = vals[q];
+  diag[4] = vals[5] - mean;
+  diag[5] = vals[6] - mean;
+  bool finite = true;
+#pragma unroll
+  for (int q = 0; q < 7; ++q) finite = finite && isfinite(vals[q]);
   double flag = diag[14];
   if (!finite) flag = fmax(flag, 1.0);
-  else if (umax_limit > 0.0 && mu > umax_limit) flag = fmax(flag, 2.0);
+  else if (umax_limit > 0.0 && vals[0] > umax_limit) flag = fmax(flag, 2.0);
   diag[14] = flag;
 }
 

@@ -307,9 +307,9 @@ __global__ void __launch_bounds__(R * NZ / KC, SlowXt<NZ, R, KC, PROD>::per_sm) 
   // per-level constants of the production components (one cell per thread)
   const float spa = spg ? (float)s.sp_a[kb] : 0.0f, spah = spg ? (float)s.sp_ah[kb] : 0.0f;
   const float spal = spg ? (float)s.sp_ah[NZ] : 0.0f;  // the lid's
-  const float dragk = drg ? (float)(s.drag_cd / s.drag_dz * s.drag_w[kb]) : 0.0f;
-  const float dnu = (float)s.diff_nu, rdx2 = (float)(1.0 / s.diff_dx2),
-              rdy2 = (float)(1.0 / s.diff_dy2);
+  const float dragk = drg ? (float)(s.drag_rate * s.drag_w[kb]) : 0.0f;
+  const float dnu = (float)s.diff_nu, rdx2 = (float)s.diff_rdx2,
+              rdy2 = (float)s.diff_rdy2;
   // planes 0..2 are read only here; 7 and 8 refill the slots of 0 and 1
 #pragma unroll
   for (int q = 0; q < 3; ++q) release(q);
