@@ -2631,22 +2631,29 @@ int oracle_b200_track_vorticity(OracleTracker* t, const void* u, const void* v, 
 
 /* ---- vortex diagnostics ------------------------------------------------- */
 
+// Results of the read-outs, in page-locked memory the kernels write: a call ends
+// with its stream's completion, without a copy back.
+struct VdResults {
+  VdMax best;
+  double sum, ring[3 * (kVdMaxBins + 1)], cen[3];
+};
+
 struct OracleVortexDiag {
   int nx = 0, ny = 0, nz = 0;
   int nblk = 1;  // CTAs of the grid-wide reductions
   int* lev = nullptr;
   double *um = nullptr, *vm = nullptr, *zeta = nullptr, *zp = nullptr, *zs = nullptr;
-  double *sq = nullptr, *dsum = nullptr, *ring = nullptr, *edges = nullptr, *cen = nullptr;
-  VdMax *part = nullptr, *best = nullptr;
+  double* sq = nullptr;
+  VdMax* part = nullptr;
+  VdResults *res = nullptr, *dres = nullptr;  // host and device addresses
   std::vector<void*> allocs;
 };
 
 namespace {
 
-constexpr int kVdMaxBins = 64;
-
 void vdiag_free(OracleVortexDiag* d) {
   for (void* q : d->allocs) cudaFree(q);
+  if (d->res) cudaFreeHost(d->res);
   delete d;
 }
 
@@ -2659,24 +2666,33 @@ int vdiag_call(const OracleVortexDiag* d, int precision, const void* u, const vo
 }
 
 // Uploads the level list after checking it is ascending inside [0, nz).
-int vdiag_levels(OracleVortexDiag* d, const int* lev, int nlev, cudaStream_t st) {
+// The band of an ascending level list; a list without gaps needs no upload.
+int vdiag_levels(OracleVortexDiag* d, const int* lev, int nlev, VdBand* band, cudaStream_t st) {
   if (!lev || nlev < 1 || nlev > d->nz) return fail(OB_ERR_ARG, "vdiag: bad level list");
   for (int l = 0; l < nlev; ++l)
     if (lev[l] < 0 || lev[l] >= d->nz || (l > 0 && lev[l] <= lev[l - 1]))
       return fail(OB_ERR_ARG, "vdiag: levels must ascend inside [0, nz)");
-  OB_CUDA(cudaMemcpyAsync(d->lev, lev, nlev * sizeof(int), cudaMemcpyHostToDevice, st));
+  band->first = lev[0];
+  band->n = nlev;
+  band->dn = FastDiv((unsigned)nlev);
+  band->lev = nullptr;
+  if (lev[nlev - 1] - lev[0] != nlev - 1) {
+    OB_CUDA(cudaMemcpyAsync(d->lev, lev, nlev * sizeof(int), cudaMemcpyHostToDevice, st));
+    band->lev = d->lev;
+  }
   return OB_OK;
 }
 
-int vdiag_mean_winds(OracleVortexDiag* d, const void* u, const void* v, int precision, int nlev,
-                     cudaStream_t st) {
+int vdiag_mean_winds(OracleVortexDiag* d, const void* u, const void* v, int precision,
+                     const VdBand& band, cudaStream_t st) {
   const long long ncol = (long long)d->nx * d->ny;
+  const unsigned nb = (unsigned)((2 * ncol + kVdThreads - 1) / kVdThreads);
   if (precision == OB_PREC_F64)
-    k_vd_band_mean<double><<<d->nblk, kVdThreads, 0, st>>>(
-        (const double*)u, (const double*)v, ncol, d->nz, d->lev, nlev, d->um, d->vm);
+    k_vd_band_mean<double><<<nb, kVdThreads, 0, st>>>((const double*)u, (const double*)v, ncol,
+                                                      d->nz, band, d->um, d->vm);
   else
-    k_vd_band_mean<float><<<d->nblk, kVdThreads, 0, st>>>(
-        (const float*)u, (const float*)v, ncol, d->nz, d->lev, nlev, d->um, d->vm);
+    k_vd_band_mean<float><<<nb, kVdThreads, 0, st>>>((const float*)u, (const float*)v, ncol,
+                                                     d->nz, band, d->um, d->vm);
   OB_LAUNCHED();
   return OB_OK;
 }
@@ -2698,7 +2714,7 @@ int oracle_b200_vdiag_create(int nx, int ny, int nz, OracleVortexDiag** out) {
   d->ny = ny;
   d->nz = nz;
   const long long ncol = (long long)nx * ny;
-  d->nblk = (int)std::min<long long>((ncol + kVdThreads - 1) / kVdThreads, 2LL * nsm);
+  d->nblk = (int)std::min<long long>((ncol + kVdThreads - 1) / kVdThreads, 8LL * nsm);
   auto A = [&](void** q, size_t bytes) {
     void* p = nullptr;
     if (cudaMalloc(&p, bytes) != cudaSuccess) return fail(OB_ERR_CUDA, "vdiag_create: cudaMalloc");
@@ -2710,13 +2726,15 @@ int oracle_b200_vdiag_create(int nx, int ny, int nz, OracleVortexDiag** out) {
   if ((rc = A((void**)&d->lev, nz * sizeof(int))) || (rc = A((void**)&d->um, ncol * 8)) ||
       (rc = A((void**)&d->vm, ncol * 8)) || (rc = A((void**)&d->zeta, ncol * 8)) ||
       (rc = A((void**)&d->zp, ncol * 8)) || (rc = A((void**)&d->zs, ncol * 8)) ||
-      (rc = A((void**)&d->sq, d->nblk * 8)) || (rc = A((void**)&d->dsum, 8)) ||
-      (rc = A((void**)&d->ring, 3 * (kVdMaxBins + 1) * 8)) ||
-      (rc = A((void**)&d->edges, (kVdMaxBins + 1) * 8)) || (rc = A((void**)&d->cen, 3 * 8)) ||
-      (rc = A((void**)&d->part, d->nblk * sizeof(VdMax))) ||
-      (rc = A((void**)&d->best, sizeof(VdMax)))) {
+      (rc = A((void**)&d->sq, d->nblk * 8)) ||
+      (rc = A((void**)&d->part, d->nblk * sizeof(VdMax)))) {
     vdiag_free(d);
     return rc;
+  }
+  if (cudaHostAlloc((void**)&d->res, sizeof(VdResults), cudaHostAllocMapped) != cudaSuccess ||
+      cudaHostGetDevicePointer((void**)&d->dres, d->res, 0) != cudaSuccess) {
+    vdiag_free(d);
+    return fail(OB_ERR_CUDA, "vdiag_create: page-locked results");
   }
   *out = d;
   return OB_OK;
@@ -2734,19 +2752,20 @@ int oracle_b200_vdiag_speed_max(OracleVortexDiag* d, const void* u, const void* 
   if (!out) return fail(OB_ERR_ARG, "vdiag_speed_max: out is NULL");
   static_assert(sizeof(VdMax) == sizeof(OracleVdMax), "VdMax layout");
   cudaStream_t st = (cudaStream_t)stream;
-  if (int rc = vdiag_levels(d, levels, nlev, st)) return rc;
+  VdBand band;
+  if (int rc = vdiag_levels(d, levels, nlev, &band, st)) return rc;
   const long long ncol = (long long)d->nx * d->ny;
   if (precision == OB_PREC_F64)
     k_vd_speed_max<double><<<d->nblk, kVdThreads, 0, st>>>(
-        (const double*)u, (const double*)v, ncol, d->nz, d->lev, nlev, u_env, v_env, d->part);
+        (const double*)u, (const double*)v, ncol, d->nz, band, u_env, v_env, d->part);
   else
     k_vd_speed_max<float><<<d->nblk, kVdThreads, 0, st>>>(
-        (const float*)u, (const float*)v, ncol, d->nz, d->lev, nlev, u_env, v_env, d->part);
+        (const float*)u, (const float*)v, ncol, d->nz, band, u_env, v_env, d->part);
   OB_LAUNCHED();
-  k_vd_max_final<<<1, kVdThreads, 0, st>>>(d->part, d->nblk, d->best);
+  k_vd_final<<<1, kVdThreads, 0, st>>>(d->part, nullptr, d->nblk, &d->dres->best, nullptr);
   OB_LAUNCHED();
-  OB_CUDA(cudaMemcpyAsync(out, d->best, sizeof(VdMax), cudaMemcpyDeviceToHost, st));
   OB_CUDA(cudaStreamSynchronize(st));
+  std::memcpy(out, &d->res->best, sizeof(VdMax));
   return OB_OK;
 }
 
@@ -2758,18 +2777,17 @@ int oracle_b200_vdiag_vorticity(OracleVortexDiag* d, const void* u, const void* 
   if (!center || !zeta_sq_sum || !(dx > 0.0) || !(dy > 0.0))
     return fail(OB_ERR_ARG, "vdiag_vorticity: bad output or spacing");
   cudaStream_t st = (cudaStream_t)stream;
-  if (int rc = vdiag_levels(d, levels, nlev, st)) return rc;
-  if (int rc = vdiag_mean_winds(d, u, v, precision, nlev, st)) return rc;
+  VdBand band;
+  if (int rc = vdiag_levels(d, levels, nlev, &band, st)) return rc;
+  if (int rc = vdiag_mean_winds(d, u, v, precision, band, st)) return rc;
   k_vd_zeta<<<d->nblk, kVdThreads, 0, st>>>(d->um, d->vm, d->nx, d->ny, dx, dy, cx_m, cy_m,
                                             window_m, d->zeta, d->part, d->sq);
   OB_LAUNCHED();
-  k_vd_max_final<<<1, kVdThreads, 0, st>>>(d->part, d->nblk, d->best);
+  k_vd_final<<<1, kVdThreads, 0, st>>>(d->part, d->sq, d->nblk, &d->dres->best, &d->dres->sum);
   OB_LAUNCHED();
-  k_vd_sum_final<<<1, kVdThreads, 0, st>>>(d->sq, d->nblk, d->dsum);
-  OB_LAUNCHED();
-  OB_CUDA(cudaMemcpyAsync(center, d->best, sizeof(VdMax), cudaMemcpyDeviceToHost, st));
-  OB_CUDA(cudaMemcpyAsync(zeta_sq_sum, d->dsum, sizeof(double), cudaMemcpyDeviceToHost, st));
   OB_CUDA(cudaStreamSynchronize(st));
+  std::memcpy(center, &d->res->best, sizeof(VdMax));
+  *zeta_sq_sum = d->res->sum;
   return OB_OK;
 }
 
@@ -2786,10 +2804,10 @@ int oracle_b200_vdiag_ke(OracleVortexDiag* d, const void* u, const void* v, int 
     k_vd_ke<float><<<d->nblk, kVdThreads, 0, st>>>((const float*)u, (const float*)v, n, u_env,
                                                    v_env, d->sq);
   OB_LAUNCHED();
-  k_vd_sum_final<<<1, kVdThreads, 0, st>>>(d->sq, d->nblk, d->dsum);
+  k_vd_final<<<1, kVdThreads, 0, st>>>(nullptr, d->sq, d->nblk, nullptr, &d->dres->sum);
   OB_LAUNCHED();
-  OB_CUDA(cudaMemcpyAsync(sum, d->dsum, sizeof(double), cudaMemcpyDeviceToHost, st));
   OB_CUDA(cudaStreamSynchronize(st));
+  *sum = d->res->sum;
   return OB_OK;
 }
 
@@ -2802,8 +2820,9 @@ int oracle_b200_vdiag_rings(OracleVortexDiag* d, const void* u, const void* v,
     return fail(OB_ERR_ARG, "vdiag_rings: bad output, edges, bin count (1..%d) or spacing",
                 kVdMaxBins);
   cudaStream_t st = (cudaStream_t)stream;
-  if (int rc = vdiag_levels(d, levels, nlev, st)) return rc;
-  if (int rc = vdiag_mean_winds(d, u, v, precision, nlev, st)) return rc;
+  VdBand band;
+  if (int rc = vdiag_levels(d, levels, nlev, &band, st)) return rc;
+  if (int rc = vdiag_mean_winds(d, u, v, precision, band, st)) return rc;
   // bounding box of the disk, one cell of margin each side (every cell with
   // r < r_vent lies inside it); empty for a non-finite centre or radius
   double rmax = r_vent_m;
@@ -2820,14 +2839,13 @@ int oracle_b200_vdiag_rings(OracleVortexDiag* d, const void* u, const void* v,
     i0 = i1 = 0;
     j0 = j1 = 0;
   }
-  OB_CUDA(cudaMemcpyAsync(d->edges, edges, (n_bins + 1) * sizeof(double),
-                          cudaMemcpyHostToDevice, st));
-  k_vd_rings<<<1, kVdThreads, 0, st>>>(d->um, d->vm, d->ny, i0, i1, j0, j1, dx, dy, cx_m, cy_m,
-                                       d->edges, n_bins, r_vent_m, d->ring);
+  VdEdges e{};
+  std::copy(edges, edges + n_bins + 1, e.r);
+  k_vd_rings<<<n_bins + 1, kVdThreads, 0, st>>>(d->um, d->vm, d->ny, i0, i1, j0, j1, dx, dy, cx_m,
+                                                cy_m, e, n_bins, r_vent_m, d->dres->ring);
   OB_LAUNCHED();
-  OB_CUDA(cudaMemcpyAsync(out, d->ring, 3 * (n_bins + 1) * sizeof(double),
-                          cudaMemcpyDeviceToHost, st));
   OB_CUDA(cudaStreamSynchronize(st));
+  std::memcpy(out, d->res->ring, 3 * (n_bins + 1) * sizeof(double));
   return OB_OK;
 }
 
@@ -2857,10 +2875,10 @@ int oracle_b200_vdiag_centroid(OracleVortexDiag* d, int i0, int i1, int j0, int 
   if (i0 < 0 || j0 < 0 || i1 > d->nx || j1 > d->ny || i1 < i0 || j1 < j0)
     return fail(OB_ERR_ARG, "vdiag_centroid: patch outside the grid");
   cudaStream_t st = (cudaStream_t)stream;
-  k_vd_centroid<<<1, kVdThreads, 0, st>>>(d->zs, d->ny, i0, i1, j0, j1, d->cen);
+  k_vd_centroid<<<1, kVdThreads, 0, st>>>(d->zs, d->ny, i0, i1, j0, j1, d->dres->cen);
   OB_LAUNCHED();
-  OB_CUDA(cudaMemcpyAsync(out, d->cen, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
   OB_CUDA(cudaStreamSynchronize(st));
+  std::memcpy(out, d->res->cen, 3 * sizeof(double));
   return OB_OK;
 }
 

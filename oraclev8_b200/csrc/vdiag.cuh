@@ -82,14 +82,6 @@ __device__ double vd_block_sum(double s) {
   return s;
 }
 
-// |(u - u_env, v - v_env)| as NumPy forms it: each square rounded, then added.
-template <class T>
-__device__ __forceinline__ double vd_speed(const T* __restrict__ u, const T* __restrict__ v,
-                                           long long o, double ue, double ve) {
-  const double up = (double)u[o] - ue, vp = (double)v[o] - ve;
-  return sqrt(__dadd_rn(__dmul_rn(up, up), __dmul_rn(vp, vp)));
-}
-
 // Cell-centre distance from (cx, cy): x = (ix + 0.5) dx, no periodic wrap
 // (diagnostics.py:40-50).
 __device__ __forceinline__ double vd_radius(int ix, int iy, double dx, double dy, double cx,
@@ -99,57 +91,136 @@ __device__ __forceinline__ double vd_radius(int ix, int iy, double dx, double dy
   return sqrt(__dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)));
 }
 
-// Per-CTA argmax partial of the perturbation speed over the listed levels
-// (ascending) of every column; the flat index is (col * nz + k).
-template <class T>
-__global__ void __launch_bounds__(kVdThreads) k_vd_speed_max(
-    const T* __restrict__ u, const T* __restrict__ v, long long ncol, int nz,
-    const int* __restrict__ lev, int nlev, double ue, double ve, VdMax* __restrict__ part) {
+// The listed levels of a reduction: lev null, first .. first + n - 1.
+struct VdBand {
+  const int* lev;
+  int first, n;
+  FastDiv dn;  // by n
+  __device__ __forceinline__ int at(int l) const { return lev ? lev[l] : first + l; }
+};
+
+// Running argmax of a thread whose indices ascend: the square decides whether
+// the root is taken (the root is monotonic, and a later index wins no tie), which
+// leaves a few roots a thread instead of one a cell.
+struct VdSpeed {
   VdMax a{-INFINITY, 0x7fffffffffffffffLL};
-  const long long n = ncol * nlev;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long col = e / nlev;
-    const int k = lev[e - col * nlev];
-    const long long o = col * nz + k;
-    const double s = vd_speed(u, v, o, ue, ve);
+  double s2 = -INFINITY;
+  __device__ __forceinline__ void take(double up, double vp, long long o) {
+    const double q = __dadd_rn(__dmul_rn(up, up), __dmul_rn(vp, vp));
+    if (q <= s2 || isnan(a.v)) return;
+    const double s = sqrt(q);
     if (vd_beats(s, o, a.v, a.i)) {
       a.v = s;
       a.i = o;
+      s2 = q;
     }
   }
-  a = vd_block_max(a);
+};
+
+// Per-CTA argmax partial of the perturbation speed over the band's levels of
+// every column; the flat index is (col * nz + k).  Every level: 16-byte loads of
+// the flat fields (512 x 512 x 64 single: the call over
+// every level 175 -> 38 us; it took a root, a 64-bit division and a 4-byte load per
+// cell).
+template <class T>
+__global__ void __launch_bounds__(kVdThreads) k_vd_speed_max(
+    const T* __restrict__ u, const T* __restrict__ v, long long ncol, int nz, VdBand band,
+    double ue, double ve, VdMax* __restrict__ part) {
+  constexpr int V = 16 / sizeof(T);
+  struct __align__(16) Vec { T a[V]; };
+  VdSpeed m;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const bool al = ((reinterpret_cast<size_t>(u) | reinterpret_cast<size_t>(v)) & 15) == 0;
+  if (band.n == nz && al) {
+    const long long n = ncol * nz, nv = n / V;
+#pragma unroll 2
+    for (long long e = first; e < nv; e += stride) {
+      const Vec x = reinterpret_cast<const Vec*>(u)[e], y = reinterpret_cast<const Vec*>(v)[e];
+#pragma unroll
+      for (int q = 0; q < V; ++q) m.take((double)x.a[q] - ue, (double)y.a[q] - ve, e * V + q);
+    }
+    for (long long o = nv * V + first; o < n; o += stride)
+      m.take((double)u[o] - ue, (double)v[o] - ve, o);
+  } else if (ncol * band.n < 0x7fffffffLL) {
+    const int n = (int)(ncol * band.n);
+#pragma unroll 4
+    for (int e = (int)first; e < n; e += (int)stride) {
+      const int col = band.dn.div(e);
+      const long long o = (long long)col * nz + band.at(e - col * band.n);
+      m.take((double)u[o] - ue, (double)v[o] - ve, o);
+    }
+  } else {
+    for (long long e = first; e < ncol * band.n; e += stride) {
+      const long long col = e / band.n, o = col * nz + band.at((int)(e - col * band.n));
+      m.take((double)u[o] - ue, (double)v[o] - ve, o);
+    }
+  }
+  const VdMax a = vd_block_max(m.a);
   if (threadIdx.x == 0) part[blockIdx.x] = a;
 }
 
-// Final argmax over the partials, in one CTA.
-__global__ void __launch_bounds__(kVdThreads) k_vd_max_final(const VdMax* __restrict__ part,
-                                                             int npart, VdMax* __restrict__ out) {
+// Final argmax over `part` and sum over `sq` (either may be null), in one CTA, into
+// the workspace's host-mapped results.
+__global__ void __launch_bounds__(kVdThreads) k_vd_final(const VdMax* __restrict__ part,
+                                                         const double* __restrict__ sq, int npart,
+                                                         VdMax* __restrict__ best,
+                                                         double* __restrict__ sum) {
   VdMax a{-INFINITY, 0x7fffffffffffffffLL};
-  for (int b = threadIdx.x; b < npart; b += blockDim.x)
-    if (vd_beats(part[b].v, part[b].i, a.v, a.i)) a = part[b];
+  double s = 0.0;
+  for (int b = threadIdx.x; b < npart; b += blockDim.x) {
+    if (part && vd_beats(part[b].v, part[b].i, a.v, a.i)) a = part[b];
+    if (sq) s = __dadd_rn(s, sq[b]);
+  }
   a = vd_block_max(a);
-  if (threadIdx.x == 0) *out = a;
+  s = vd_block_sum(s);
+  if (threadIdx.x == 0) {
+    if (part) *best = a;
+    if (sq) *sum = s;
+  }
 }
 
-// Column means of u and v over the listed levels: a sequential sum from the
-// first listed level, divided by the count (NumPy's mean of u[:, :, band]).
+// Column means of u and v over the band's levels: a sequential sum from the
+// first one, divided by the count (NumPy's mean of u[:, :, band]).  A thread per
+// column and field; a band without gaps is read by 16 bytes, kVdAhead loads in
+// flight (48 levels of 512 x 512 x 64 single: 110 -> 28 us; a level a load, one
+// after the other, took 0.9 TB/s; staging columns in shared memory was no
+// faster, its index arithmetic costing what the lines did).
+constexpr int kVdAhead = 8;
 template <class T>
 __global__ void __launch_bounds__(kVdThreads) k_vd_band_mean(
-    const T* __restrict__ u, const T* __restrict__ v, long long ncol, int nz,
-    const int* __restrict__ lev, int nlev, double* __restrict__ um, double* __restrict__ vm) {
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < ncol;
-       c += (long long)gridDim.x * blockDim.x) {
-    const T* uc = u + c * nz;
-    const T* vc = v + c * nz;
-    double su = (double)uc[lev[0]], sv = (double)vc[lev[0]];
-    for (int l = 1; l < nlev; ++l) {
-      su = __dadd_rn(su, (double)uc[lev[l]]);
-      sv = __dadd_rn(sv, (double)vc[lev[l]]);
+    const T* __restrict__ u, const T* __restrict__ v, long long ncol, int nz, VdBand band,
+    double* __restrict__ um, double* __restrict__ vm) {
+  constexpr int V = 16 / sizeof(T);
+  struct __align__(16) Vec { T a[V]; };
+  const long long t = blockIdx.x * (long long)kVdThreads + threadIdx.x;
+  if (t >= 2 * ncol) return;
+  const bool second = t >= ncol;
+  const long long c = second ? t - ncol : t;
+  const T* col = (second ? v : u) + c * nz;
+  double s = 0.0;
+  if (!band.lev && nz % V == 0 && (reinterpret_cast<size_t>(second ? v : u) & 15) == 0) {
+    const int last = band.first + band.n - 1;
+    for (int w0 = band.first / V; w0 <= last / V; w0 += kVdAhead) {
+      Vec x[kVdAhead];
+#pragma unroll
+      for (int i = 0; i < kVdAhead; ++i)
+        if (w0 + i <= last / V) x[i] = reinterpret_cast<const Vec*>(col)[w0 + i];
+#pragma unroll
+      for (int i = 0; i < kVdAhead; ++i)
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+          const int k = (w0 + i) * V + q;
+          if (k == band.first) s = (double)x[i].a[q];
+          else if (k > band.first && k <= last) s = __dadd_rn(s, (double)x[i].a[q]);
+        }
     }
-    um[c] = su / (double)nlev;
-    vm[c] = sv / (double)nlev;
+  } else {
+    s = (double)col[band.at(0)];
+#pragma unroll 8
+    for (int l = 1; l < band.n; ++l) s = __dadd_rn(s, (double)col[band.at(l)]);
   }
+  (second ? vm : um)[c] = s / (double)band.n;
 }
 
 // zeta = (v[i+1] - v[i-1]) / (2 dx) - (u[j+1] - u[j-1]) / (2 dy), periodic
@@ -193,57 +264,63 @@ __global__ void __launch_bounds__(kVdThreads) k_vd_ke(const T* __restrict__ u,
                                                       const T* __restrict__ v, long long n,
                                                       double ue, double ve,
                                                       double* __restrict__ part) {
+  constexpr int V = 16 / sizeof(T);
+  struct __align__(16) Vec { T a[V]; };
   double s = 0.0;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    const double up = (double)u[e] - ue, vp = (double)v[e] - ve;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  auto add = [&](T a, T b) {
+    const double up = (double)a - ue, vp = (double)b - ve;
     s = __dadd_rn(s, __dadd_rn(__dmul_rn(up, up), __dmul_rn(vp, vp)));
+  };
+  const bool al = ((reinterpret_cast<size_t>(u) | reinterpret_cast<size_t>(v)) & 15) == 0;
+  const long long nv = al ? n / V : 0;
+#pragma unroll 4
+  for (long long e = first; e < nv; e += stride) {
+    const Vec x = reinterpret_cast<const Vec*>(u)[e], y = reinterpret_cast<const Vec*>(v)[e];
+#pragma unroll
+    for (int q = 0; q < V; ++q) add(x.a[q], y.a[q]);
   }
+  for (long long e = nv * V + first; e < n; e += stride) add(u[e], v[e]);
   s = vd_block_sum(s);
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-// Sum of the partials in one CTA (fixed order).
-__global__ void __launch_bounds__(kVdThreads) k_vd_sum_final(const double* __restrict__ part,
-                                                             int npart, double* __restrict__ out) {
-  double s = 0.0;
-  for (int b = threadIdx.x; b < npart; b += blockDim.x) s = __dadd_rn(s, part[b]);
-  s = vd_block_sum(s);
-  if (threadIdx.x == 0) *out = s;
-}
+constexpr int kVdMaxBins = 64;  // ventilation rings (header: 1 <= n_bins <= 64)
+struct VdEdges {
+  double r[kVdMaxBins + 1];
+};
 
 // Ring sums of the deep-layer winds for the ventilation flow
-// (diagnostics.py:150-166), one CTA over the disk's bounding box
+// (diagnostics.py:150-166), a CTA per ring over the disk's bounding box
 // [i0, i1) x [j0, j1).  out[3 b + 0..2] = (cells, sum u, sum v) of ring b
 // (edges[b] <= r < edges[b + 1]); ring nb is the disk r < r_vent.
 __global__ void __launch_bounds__(kVdThreads) k_vd_rings(
     const double* __restrict__ um, const double* __restrict__ vm, int ny, int i0, int i1,
     int j0, int j1, double dx, double dy, double cx, double cy,
-    const double* __restrict__ edges, int nb, double r_vent, double* __restrict__ out) {
-  const int bw = j1 - j0;
+    const __grid_constant__ VdEdges edges, int nb, double r_vent, double* __restrict__ out) {
+  const int bw = j1 - j0, b = blockIdx.x;
   const long long nbox = (long long)(i1 - i0) * bw;
-  for (int b = 0; b <= nb; ++b) {
-    const double lo = b < nb ? edges[b] : -INFINITY;
-    const double hi = b < nb ? edges[b + 1] : r_vent;
-    double cnt = 0.0, su = 0.0, sv = 0.0;
-    for (long long e = threadIdx.x; e < nbox; e += blockDim.x) {
-      const int ix = i0 + (int)(e / bw), iy = j0 + (int)(e % bw);
-      const double r = vd_radius(ix, iy, dx, dy, cx, cy);
-      if (r >= lo && r < hi) {
-        const long long c = (long long)ix * ny + iy;
-        cnt += 1.0;
-        su = __dadd_rn(su, um[c]);
-        sv = __dadd_rn(sv, vm[c]);
-      }
+  const double lo = b < nb ? edges.r[b] : -INFINITY;
+  const double hi = b < nb ? edges.r[b + 1] : r_vent;
+  double cnt = 0.0, su = 0.0, sv = 0.0;
+  for (long long e = threadIdx.x; e < nbox; e += blockDim.x) {
+    const int ix = i0 + (int)(e / bw), iy = j0 + (int)(e % bw);
+    const double r = vd_radius(ix, iy, dx, dy, cx, cy);
+    if (r >= lo && r < hi) {
+      const long long c = (long long)ix * ny + iy;
+      cnt += 1.0;
+      su = __dadd_rn(su, um[c]);
+      sv = __dadd_rn(sv, vm[c]);
     }
-    cnt = vd_block_sum(cnt);
-    su = vd_block_sum(su);
-    sv = vd_block_sum(sv);
-    if (threadIdx.x == 0) {
-      out[3 * b + 0] = cnt;
-      out[3 * b + 1] = su;
-      out[3 * b + 2] = sv;
-    }
+  }
+  cnt = vd_block_sum(cnt);
+  su = vd_block_sum(su);
+  sv = vd_block_sum(sv);
+  if (threadIdx.x == 0) {
+    out[3 * b + 0] = cnt;
+    out[3 * b + 1] = su;
+    out[3 * b + 2] = sv;
   }
 }
 

@@ -258,9 +258,12 @@ def compute_diagnostics(state, base, cx_m, cy_m, dx, dy, u_env=0.0, v_env=0.0,
                         theta_xy_m=None, r_vent_m=120e3):
     """All read-outs, anchored on the vorticity centre (diagnostics.py:226-254)."""
     d = {}
-    vc = vorticity_center(state, cx_m, cy_m, dx, dy, base=base)
-    d.update(vc)
-    cxv, cyv = vc["xv_m"], vc["yv_m"]
+    nx, ny = int(state.u.shape[0]), int(state.u.shape[1])
+    # vorticity_center and enstrophy read the same low-level vorticity
+    flat, zeta_sq = _vorticity(state, base, dx, dy, cx_m, cy_m, 200e3, 3000.0)
+    ix, iy = divmod(flat, ny)
+    cxv, cyv = float(_centres(ix, dx)), float(_centres(iy, dy))
+    d.update(xv_m=cxv, yv_m=cyv)
     d.update(low_level_vmax(state, base, cxv, cyv, dx, dy, u_env, v_env))
     d.update(vmax_3d(state, base, u_env, v_env))
     d.update(ventilation_flow(state, cxv, cyv, dx, dy, base=base, r_vent_m=r_vent_m,
@@ -268,7 +271,7 @@ def compute_diagnostics(state, base, cx_m, cy_m, dx, dy, u_env=0.0, v_env=0.0,
     if theta_xy_m is not None:
         d["sep_km"] = center_separation_km(theta_xy_m, (cxv, cyv))
     d.update(perturbation_ke(state, u_env, v_env))
-    d.update(enstrophy(state, dx, dy, base=base))
+    d["enstrophy"] = float(0.5 * (zeta_sq / (nx * ny)))
     return d
 
 
