@@ -1729,6 +1729,44 @@ bool slow_xt_launch_any(OraclePlan* p, int mask, double dts, const float* u, con
   return false;
 }
 
+// ---- x-marching slow tendency over planes that the threads load (k_slow_xw)
+// Grids of nx >= 7 and ny >= 10: a halo row or column wraps at most once.
+// Smaller ones, and plans whose slow_xw is 0, take the gather form.
+template <class T, int OUT, int H, bool PROD>
+void slow_xw_launch(OraclePlan* p, int mask, double dts, const T* u, const T* v, const T* w,
+                    const T* th, T* uo, T* vo, T* wo, T* tho, cudaStream_t st) {
+  const int nx = p->g.nx, nk = (p->g.nz + 31) / 32, kw = (p->g.nz + nk - 1) / nk;
+  const int nrow = (p->g.ny + kXwTJ - 1) / kXwTJ;
+  int dev = 0, nsm = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  // segments: four CTAs per SM where the grid gives them, 7 to 35 columns
+  // (each segment loads its window's 2 H columns again)
+  const int want = std::max(1, 4 * nsm / (nrow * nk));
+  const int seg = std::min(35, std::max(7, ((nx + want - 1) / want + 6) / 7 * 7));
+  const dim3 grid(nrow, (nx + seg - 1) / seg, nk);
+  const int threads = std::max(128, (kXwTJ * kw + 31) / 32 * 32);
+  k_slow_xw<T, OUT, H, PROD><<<grid, threads, 0, st>>>(p->g, slow_args(p), mask, dts, seg, kw, u,
+                                                       v, w, th, (const T*)p->Du,
+                                                       (const T*)p->Dv, uo, vo, wo, tho);
+}
+template <class T, int OUT>
+bool slow_xw_launch_any(OraclePlan* p, int mask, double dts, bool prod, const T* u, const T* v,
+                        const T* w, const T* th, T* uo, T* vo, T* wo, T* tho, cudaStream_t st) {
+  if (!p->slow_xw || p->g.nx < 7 || p->g.ny < 10) return false;
+  const bool ws5 = (mask & OB_TEND_ADVECTION) && p->advection == OB_ADV_UPWIND5H;
+  Launch L_(p, 5, st);
+  if (ws5 && prod)
+    slow_xw_launch<T, OUT, 3, true>(p, mask, dts, u, v, w, th, uo, vo, wo, tho, st);
+  else if (ws5)
+    slow_xw_launch<T, OUT, 3, false>(p, mask, dts, u, v, w, th, uo, vo, wo, tho, st);
+  else if (prod)
+    slow_xw_launch<T, OUT, 1, true>(p, mask, dts, u, v, w, th, uo, vo, wo, tho, st);
+  else
+    slow_xw_launch<T, OUT, 1, false>(p, mask, dts, u, v, w, th, uo, vo, wo, tho, st);
+  return true;
+}
+
 template <class T, int OUT>
 int slow_impl(OraclePlan* p, int mask, double dts, const T* u, const T* v, const T* w,
               const T* th, T* uo, T* vo, T* wo, T* tho, cudaStream_t st) {
@@ -1741,28 +1779,37 @@ int slow_impl(OraclePlan* p, int mask, double dts, const T* u, const T* v, const
           p->g, u, v, 1.0 / p->diff_dx2, 1.0 / p->diff_dy2, (T*)p->Lu, (T*)p->Lv); }
     OB_LAUNCHED();
   }
-  // production components run in the gather kernels
   const bool extra = (mask & (OB_TEND_DRAG | OB_TEND_SPONGE | OB_TEND_DIFFUSION | OB_TEND_COOLING)) &&
                      (p->drag || p->sponge || p->diffusion || p->cooling);
+  // the bulk-copied planes where the grid tiles them, else the plain march,
+  // and the gather on grids too small for it
   if constexpr (sizeof(T) == 4) {
-    // the x-marching form where the grid tiles it; the gather form otherwise
-    if (slow_xt_call(p, mask, u, v, w, th))
+    if (slow_xt_call(p, mask, u, v, w, th)) {
       { Launch L_(p, 5, st); slow_xt_launch_any<OUT>(p, mask, dts, u, v, w, th, uo, vo, wo, tho, st); }
-    else if (p->slow_xw && !extra && p->g.ny % 8 == 0 && p->g.nx % KXW == 0)
-      { Launch L_(p, 5, st); k_slow_xw<OUT><<<dim3(p->g.ny / 8, p->g.nx / KXW), blk, 0, st>>>(
-            p->g, slow_args(p), mask, dts, u, v, w, th, (const T*)p->Du, (const T*)p->Dv, uo, vo, wo, tho); }
-    else if (extra)
-      { Launch L_(p, 5, st); k_slow_f32<OUT, true><<<grd, blk, 0, st>>>(p->g, slow_args(p), mask, dts, u, v, w, th, (const T*)p->Du,
-                                                  (const T*)p->Dv, uo, vo, wo, tho); }
+      OB_LAUNCHED();
+      return OB_OK;
+    }
+  }
+  if (slow_xw_launch_any<T, OUT>(p, mask, dts, extra, u, v, w, th, uo, vo, wo, tho, st)) {
+    OB_LAUNCHED();
+    return OB_OK;
+  }
+  const T* du = (const T*)p->Du;
+  const T* dv = (const T*)p->Dv;
+  Launch L_(p, 5, st);
+  if constexpr (sizeof(T) == 4) {
+    if (extra)
+      k_slow_f32<OUT, true><<<grd, blk, 0, st>>>(p->g, slow_args(p), mask, dts, u, v, w, th, du,
+                                                 dv, uo, vo, wo, tho);
     else
-      { Launch L_(p, 5, st); k_slow_f32<OUT><<<grd, blk, 0, st>>>(p->g, slow_args(p), mask, dts, u, v, w, th, (const T*)p->Du,
-                                            (const T*)p->Dv, uo, vo, wo, tho); }
+      k_slow_f32<OUT><<<grd, blk, 0, st>>>(p->g, slow_args(p), mask, dts, u, v, w, th, du, dv,
+                                           uo, vo, wo, tho);
   } else if (extra) {
-    { Launch L_(p, 5, st); k_slow<T, OUT, true><<<grd, blk, 0, st>>>(p->g, slow_args(p), mask, dts, u, v, w, th, (const T*)p->Du,
-                                              (const T*)p->Dv, uo, vo, wo, tho); }
+    k_slow<T, OUT, true><<<grd, blk, 0, st>>>(p->g, slow_args(p), mask, dts, u, v, w, th, du, dv,
+                                              uo, vo, wo, tho);
   } else {
-    { Launch L_(p, 5, st); k_slow<T, OUT><<<grd, blk, 0, st>>>(p->g, slow_args(p), mask, dts, u, v, w, th, (const T*)p->Du,
-                                        (const T*)p->Dv, uo, vo, wo, tho); }
+    k_slow<T, OUT><<<grd, blk, 0, st>>>(p->g, slow_args(p), mask, dts, u, v, w, th, du, dv, uo,
+                                        vo, wo, tho);
   }
   OB_LAUNCHED();
   return OB_OK;

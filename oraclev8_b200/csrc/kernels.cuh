@@ -1262,252 +1262,291 @@ __global__ void __launch_bounds__(256, PROD ? 5 : 4) k_slow_f32(GridK g, SlowK s
   }
 }
 
-// k_slow_f32 marching along x.  A CTA covers TJ = 8 rows j, a z-chunk of 32
-// levels at a time, and KXW consecutive x cells.  Each thread keeps, for its
-// (j, k), a 7-point window of u, v, theta', w along x in registers (the x
-// stencils' points; one new column loaded per step), and the CTA shares, per
-// x step, a plane of the four fields over its rows plus three halo rows on
-// either side and one halo level above and below (the y and z neighbours),
-// double-buffered so that one barrier per step suffices.  Global loads per
-// cell: about 7, against about 48 gathered loads of k_slow_f32, whose x
-// neighbours come from the columns other CTAs own (seven L2 reads of every
-// value).  Same arithmetic, terms and order as k_slow_f32.
-// Requires ny % 8 == 0 and nx % KXW == 0.  grid = (ny / 8, nx / KXW),
-// block = (32, 8).
-constexpr int KXW = 16;
-constexpr int kXwRows = 8 + 6;   // plane rows: j0-3 .. j0+10
+// k_slow / k_slow_f32 marching along x, for any grid with nx >= 7 and
+// ny >= 10.  A CTA covers 8 rows j, kw <= 32 levels (the column in equal
+// chunks, so that nz = 45 runs as 23 + 22 and not as 32 + 13) and `seg`
+// consecutive x cells.  Each thread keeps, for its (j, k), a window of u, v,
+// theta', w along x in registers (2 H + 1 points; one new column loaded per
+// step), and the CTA shares, per x step, a plane of the four fields over its
+// rows plus H halo rows on either side and one halo level above and below
+// (the y and z neighbours), double-buffered so that one barrier per step
+// suffices.  H = 3: WS5 advection; H = 1: centred or none.
+// What bounds it: the gather forms wait on ~48 loads a cell, whose x and y
+// neighbours other CTAs own too; this one loads about 7 and waits on the
+// arithmetic and the shared-memory reads of the y stencils (24 a cell) at the
+// 16 (double) or 24 warps per SM its windows leave.  Two steps a turn of the
+// loop halve the moves of the window's rotation (seven, which would make it a
+// renaming, spill in double precision).  Same terms and order as the gather
+// forms.  Gather against march, a slow half (us): 512 x 512 x 64 double, WS5,
+// 640 -> 405; 320 x 320 x 32 double, production, 198 -> 141; 360 x 300 x 60
+// single, WS5, 133 -> 126.
+// grid = (ceil(ny / 8), ceil(nx / seg), ceil(nz / kw)); block: at least
+// max(8 kw, 128) threads.
+constexpr int kXwTJ = 8;         // rows per CTA
 constexpr int kXwCols = 32 + 2;  // plane columns: k0-1 .. k0+32
 
-__device__ __forceinline__ float ws5_win(const float (&q)[7], float a, float inv60d) {
-  // q[r] = value at offset r - 3
-  const bool up = a >= 0.0f;
-  const float m3 = up ? q[0] : q[6], m2 = up ? q[1] : q[5], m1 = up ? q[2] : q[4];
-  const float p1 = up ? q[4] : q[2], p2 = up ? q[5] : q[1];
-  const float d = -2.0f * m3 + 15.0f * m2 - 60.0f * m1 + 20.0f * q[3] + 30.0f * p1 - 3.0f * p2;
+// values at offsets -3 .. 3 of q (window) or of column c (plane, row stride kXwCols)
+template <class T>
+__device__ __forceinline__ T ws5_win(const T (&q)[7], T a, T inv60d) {
+  const bool up = a >= (T)0;
+  const T m3 = up ? q[0] : q[6], m2 = up ? q[1] : q[5], m1 = up ? q[2] : q[4];
+  const T p1 = up ? q[4] : q[2], p2 = up ? q[5] : q[1];
+  const T d = (T)-2 * m3 + (T)15 * m2 - (T)60 * m1 + (T)20 * q[3] + (T)30 * p1 - (T)3 * p2;
   return (up ? d : -d) * inv60d;
 }
-// the same over plane column c: rows r0-3 .. r0+3, row stride kXwCols
-__device__ __forceinline__ float ws5_col(const float* P, int r0, int c, float a, float inv60d) {
-  const bool up = a >= 0.0f;
+template <class T>
+__device__ __forceinline__ T ws5_col(const T* q, T a, T inv60d) {
+  const bool up = a >= (T)0;
   const int s = up ? kXwCols : -kXwCols;
-  const float* q = P + r0 * kXwCols + c;
-  const float d = -2.0f * q[-3 * s] + 15.0f * q[-2 * s] - 60.0f * q[-s] + 20.0f * q[0] +
-                  30.0f * q[s] - 3.0f * q[2 * s];
+  const T d = (T)-2 * q[-3 * s] + (T)15 * q[-2 * s] - (T)60 * q[-s] + (T)20 * q[0] +
+              (T)30 * q[s] - (T)3 * q[2 * s];
   return (up ? d : -d) * inv60d;
+}
+// the derivative along x (of the window) and along y (of the plane's column)
+template <int H, class T>
+__device__ __forceinline__ T xw_ddx(const T (&q)[2 * H + 1], T a, T inv) {
+  if constexpr (H == 3) return ws5_win<T>(q, a, inv);
+  else return (q[2] - q[0]) * inv;
+}
+template <int H, class T>
+__device__ __forceinline__ T xw_ddy(const T* q, T a, T inv) {
+  if constexpr (H == 3) return ws5_col<T>(q, a, inv);
+  else return (q[kXwCols] - q[-kXwCols]) * inv;
 }
 
-template <int OUTMODE>
-__global__ void __launch_bounds__(256, 3) k_slow_xw(GridK g, SlowK s, int mask, double dts_d,
-                                                    const float* __restrict__ u,
-                                                    const float* __restrict__ v,
-                                                    const float* __restrict__ w,
-                                                    const float* __restrict__ th,
-                                                    const float* __restrict__ dmp_u,
-                                                    const float* __restrict__ dmp_v,
-                                                    float* __restrict__ uo, float* __restrict__ vo,
-                                                    float* __restrict__ wo,
-                                                    float* __restrict__ tho) {
-  __shared__ float plane[2][4][kXwRows * kXwCols];
+template <class T, int OUTMODE, int H, bool PROD>
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3) k_slow_xw(
+    GridK g, SlowK s, int mask, double dts_d, int seg, int kw, const T* __restrict__ u,
+    const T* __restrict__ v, const T* __restrict__ w, const T* __restrict__ th,
+    const T* __restrict__ dmp_u, const T* __restrict__ dmp_v, T* __restrict__ uo,
+    T* __restrict__ vo, T* __restrict__ wo, T* __restrict__ tho) {
+  constexpr int WIN = 2 * H + 1;
+  constexpr int ROWS = kXwTJ + 2 * H;       // plane rows: j0-H .. j0+7+H
+  constexpr int PL = ROWS * kXwCols;
+  constexpr int NKH = 2 * ROWS;             // level-halo values per field
+  __shared__ T plane[2][4 * PL];
+  static_assert(4 * NKH <= 128, "one level-halo value a thread, 128 threads at least");
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int nzw = nz + 1;
-  const int lane = threadIdx.x, row = threadIdx.y;
-  const int tid = row * 32 + lane;
-  const int j0 = blockIdx.x * 8, j = j0 + row;
-  const int i0 = blockIdx.y * KXW;
-  const int r0 = row + 3;  // own plane row
+  const int tid = threadIdx.x;
+  const int row = tid / kw, lane = tid - row * kw;
+  const bool mine = row < kXwTJ;            // threads past 8 kw only load level halos
+  const int k0 = blockIdx.z * kw, k = k0 + lane;
+  const bool kin = mine && k < nz, win_ = mine && k <= nz;
+  auto wrap_y = [&](int j_) {
+    j_ += (j_ < 0) ? ny : 0;
+    return j_ - ((j_ >= ny) ? ny : 0);
+  };
+  const int j0 = blockIdx.x * kXwTJ;
+  const bool jin = j0 + row < ny;           // rows past ny hold the wrapped halo
+  const int j = wrap_y(j0 + (mine ? row : 0));
+  const int i0 = blockIdx.y * seg;
+  const int nstep = min(seg, nx - i0);
   const bool adv = (mask & 1) && s.adv;
   const bool cor = (mask & 2) && s.cor;
   const bool dmp = (mask & 4) && s.damp;
   const bool heat = (mask & 8) && s.heat;
-  const bool ws5 = (s.adv == 2);
-  const float dts = (float)dts_d;
-  const float inv60dx = (float)s.inv60dx, inv60dy = (float)s.inv60dy;
-  const float inv2dx = (float)s.inv2dx, inv2dy = (float)s.inv2dy;
-  const float inv2dz = (float)s.inv2dz, invdz = (float)s.invdz;
-  const float f = cor ? (float)((s.cor == 2) ? s.fy[j] : s.f0) : 0.0f;
-  const float u_env = (float)s.u_env, v_env = (float)s.v_env;
-  // halo row this thread loads (rows 0-2: j0-3..j0-1, rows 5-7: j0+8..j0+10)
-  const int hrow = row < 3 ? row : (row >= 5 ? row + 6 : -1);
-  int jh = j0 - 3 + (hrow < 0 ? 0 : hrow);
-  jh += (jh < 0) ? ny : 0;
-  jh -= (jh >= ny) ? ny : 0;
-  // k-halo value this thread loads: field kf, plane row kr, end ke
-  const int kf = tid / 28, krem = tid - kf * 28, kr = krem >> 1, ke = krem & 1;
-  int jk = j0 - 3 + kr;
-  jk += (jk < 0) ? ny : 0;
-  jk -= (jk >= ny) ? ny : 0;
-  // field f: 0 u, 1 v, 2 theta', 3 w (nz + 1 levels)
-  auto fptr = [&](int f_) { return f_ == 0 ? u : (f_ == 1 ? v : th); };
+  const bool drg = PROD && (mask & kTendDrag) && s.drag;
+  const bool spg = PROD && (mask & kTendSponge) && s.sponge;
+  const int dif = (PROD && (mask & kTendDiffusion)) ? s.diff : 0;
+  const bool col_ = PROD && (mask & kTendCooling) && s.cool;
+  const T dts = (T)dts_d;
+  const T invx = (T)(H == 3 ? s.inv60dx : s.inv2dx), invy = (T)(H == 3 ? s.inv60dy : s.inv2dy);
+  const T inv2dz = (T)s.inv2dz, invdz = (T)s.invdz;
+  const T f = cor ? (T)((s.cor == 2) ? s.fy[j] : s.f0) : (T)0;
+  // halo row this thread loads: rows 0..H-1 take j0-H.., rows 8-H..7 take j0+8..
+  const int hrow = !mine ? -1 : row < H ? row : (row >= kXwTJ - H ? row + 2 * H : -1);
+  const int jh = wrap_y(j0 - H + (hrow < 0 ? 0 : hrow));
+  // level-halo value this thread loads: field kf, plane row kr, end ke
+  const bool khal = tid < 4 * NKH;
+  const int kf = khal ? tid / NKH : 0, krem = tid - kf * NKH, kr = krem >> 1, ke = krem & 1;
+  const int jk = wrap_y(j0 - H + (khal ? kr : 0));
+  const int kk = ke ? k0 + kw : k0 - 1;
+  const int klv = kf < 3 ? nz : nzw;        // levels of that field
+  const bool kld = khal && kk >= 0 && kk < klv;
+  const T* kptr = kf == 0 ? u : kf == 1 ? v : kf == 2 ? th : w;
+  const int kat = (kr * kXwCols + (ke ? kw + 1 : 0)) + kf * PL;
+  // per-level constants
+  const T dth0k = (adv && kin) ? (T)s.dth0[k] : (T)0;
+  const T heatz = (heat && kin) ? (T)s.heat_z[k] : (T)0;
+  const T dragw = (drg && kin) ? (T)s.drag_w[k] : (T)0;
+  const T spa = (spg && kin) ? (T)s.sp_a[k] : (T)0;
+  const T spah = (spg && win_) ? (T)s.sp_ah[k] : (T)0;
+  const T* lu = static_cast<const T*>(s.lap_u);
+  const T* lv = static_cast<const T*>(s.lap_v);
+  const int jm = wrap_y(j - 1), jp = wrap_y(j + 1);
 
-  for (int k0 = 0; k0 < nz; k0 += 32) {
-    const int k = k0 + lane;
-    const bool kin = k < nz;
-    // per-level constants of this thread's level, once per chunk
-    const float dth0k = (adv && kin) ? (float)s.dth0[k] : 0.0f;
-    const float heatz = (heat && kin) ? (float)s.heat_z[k] : 0.0f;
-    auto at = [&](int ii, int jj, int f_) -> float {  // cell (ii, jj, k) of field f_
-      return f_ < 3 ? fptr(f_)[(ii * ny + jj) * nz + k] : w[(ii * ny + jj) * nzw + k];
-    };
-    // the global values of step x = ii: the window's new column (x + 3), the
-    // halo row's four fields and the level-halo value at x (software
-    // pipelined: loaded one step ahead of their use)
-    float nu, nv, nt, nw, hv[4], kv;
-    auto load_step = [&](int ii) {
-      int in = ii + 3;
-      in -= (in >= nx) ? nx : 0;
-      nu = kin ? at(in, j, 0) : 0.0f;
-      nv = kin ? at(in, j, 1) : 0.0f;
-      nt = kin ? at(in, j, 2) : 0.0f;
-      nw = kin ? at(in, j, 3) : 0.0f;
-      if (hrow >= 0) {
-#pragma unroll
-        for (int f_ = 0; f_ < 4; ++f_) {
-          float val = 0.0f;
-          if (kin) val = at(ii, jh, f_);
-          else if (f_ == 3 && k == nz) val = w[(ii * ny + jh) * nzw + nz];
-          hv[f_] = val;
-        }
-      }
-      kv = 0.0f;
-      if (tid < 4 * 28) {
-        const int kk = ke ? k0 + 32 : k0 - 1;
-        const int lim = kf < 3 ? nz : nzw;
-        if (kk >= 0 && kk < lim)
-          kv = kf < 3 ? fptr(kf)[(ii * ny + jk) * nz + kk] : w[(ii * ny + jk) * nzw + kk];
-      }
-    };
-    // prefill the windows with x = i0-3 .. i0+2
-    float qu[7], qv[7], qt[7], qw[7];
-#pragma unroll
-    for (int r = 1; r < 7; ++r) {
-      int ii = i0 - 4 + r;
-      ii += (ii < 0) ? nx : 0;
-      qu[r] = kin ? at(ii, j, 0) : 0.0f;
-      qv[r] = kin ? at(ii, j, 1) : 0.0f;
-      qt[r] = kin ? at(ii, j, 2) : 0.0f;
-      qw[r] = kin ? at(ii, j, 3) : 0.0f;
-    }
-    load_step(i0);
-    for (int step = 0; step < KXW; ++step) {
-      const int i = i0 + step;
-#pragma unroll
-      for (int r = 0; r < 6; ++r) {
-        qu[r] = qu[r + 1];
-        qv[r] = qv[r + 1];
-        qt[r] = qt[r + 1];
-        qw[r] = qw[r + 1];
-      }
-      qu[6] = nu;
-      qv[6] = nv;
-      qt[6] = nt;
-      qw[6] = nw;
-      // this step's plane: own row from the window centres, halo rows and
-      // levels from the values loaded one step ahead (the lid w at level nz
-      // included)
-      float* P = &plane[step & 1][0][0];
-      const int c = lane + 1;
-      P[0 * kXwRows * kXwCols + r0 * kXwCols + c] = qu[3];
-      P[1 * kXwRows * kXwCols + r0 * kXwCols + c] = qv[3];
-      P[2 * kXwRows * kXwCols + r0 * kXwCols + c] = qt[3];
-      P[3 * kXwRows * kXwCols + r0 * kXwCols + c] =
-          kin ? qw[3] : (k == nz ? w[(i * ny + j) * nzw + nz] : 0.0f);
-      if (hrow >= 0) {
-#pragma unroll
-        for (int f_ = 0; f_ < 4; ++f_) P[f_ * kXwRows * kXwCols + hrow * kXwCols + c] = hv[f_];
-      }
-      if (tid < 4 * 28) P[kf * kXwRows * kXwCols + kr * kXwCols + (ke ? kXwCols - 1 : 0)] = kv;
-      if (step + 1 < KXW) load_step(i + 1);
-      __syncthreads();
+  // step x = ii: the window's new column (x + H) into registers, one step
+  // ahead of its use; the halo row's four fields and the level-halo value into
+  // the step's plane, asynchronously (a level past the column's end is not
+  // copied, and nothing reads its slot)
+  T nu, nv, nt, nw;
+  auto load_column = [&](int ii) {
+    int in = ii + H;
+    in -= (in >= nx) ? nx : 0;
+    const int c = in * ny + j;
+    nu = kin ? u[c * nz + k] : (T)0;
+    nv = kin ? v[c * nz + k] : (T)0;
+    nt = kin ? th[c * nz + k] : (T)0;
+    nw = win_ ? w[c * nzw + k] : (T)0;
+  };
+  auto copy_halo = [&](int ii, T* P) {
+    if (hrow >= 0) {
+      T* d = P + hrow * kXwCols + lane + 1;
+      const int ch = ii * ny + jh;
       if (kin) {
-        const float* Pu = P;
-        const float* Pv = P + kXwRows * kXwCols;
-        const float* Pt = P + 2 * kXwRows * kXwCols;
-        const float* Pw = P + 3 * kXwRows * kXwCols;
-        const int pc = r0 * kXwCols + c;
-        const int col = i * ny + j;
-        const int o = col * nz + k;
-        const int ow = col * nzw + k;
-        const float uc = qu[3], vc = qv[3], thc = qt[3];
-        float tu = 0.0f, tv = 0.0f, tt = 0.0f;
-        if (adv) {
-          const float wc = 0.5f * (Pw[pc] + Pw[pc + 1]);
-          float czu, czv, czt;
-          if (k == 0) {
-            czu = (Pu[pc + 1] - uc) * invdz;
-            czv = (Pv[pc + 1] - vc) * invdz;
-            czt = (Pt[pc + 1] - thc) * invdz;
-          } else if (k == nz - 1) {
-            czu = (uc - Pu[pc - 1]) * invdz;
-            czv = (vc - Pv[pc - 1]) * invdz;
-            czt = (thc - Pt[pc - 1]) * invdz;
-          } else {
-            czu = (Pu[pc + 1] - Pu[pc - 1]) * inv2dz;
-            czv = (Pv[pc + 1] - Pv[pc - 1]) * inv2dz;
-            czt = (Pt[pc + 1] - Pt[pc - 1]) * inv2dz;
-          }
-          float xu, yu, xv, yv, xt, yt;
-          if (ws5) {
-            xt = ws5_win(qt, uc, inv60dx);
-            yt = ws5_col(Pt, r0, c, vc, inv60dy);
-            xu = ws5_win(qu, uc, inv60dx);
-            yu = ws5_col(Pu, r0, c, vc, inv60dy);
-            xv = ws5_win(qv, uc, inv60dx);
-            yv = ws5_col(Pv, r0, c, vc, inv60dy);
-          } else {
-            xt = (qt[4] - qt[2]) * inv2dx;
-            yt = (Pt[pc + kXwCols] - Pt[pc - kXwCols]) * inv2dy;
-            xu = (qu[4] - qu[2]) * inv2dx;
-            yu = (Pu[pc + kXwCols] - Pu[pc - kXwCols]) * inv2dy;
-            xv = (qv[4] - qv[2]) * inv2dx;
-            yv = (Pv[pc + kXwCols] - Pv[pc - kXwCols]) * inv2dy;
-          }
-          tt = -(uc * xt + vc * yt + wc * (czt + dth0k));
-          tu = -(uc * xu + vc * yu + wc * czu);
-          tv = -(uc * xv + vc * yv + wc * czv);
-        }
-        if (cor) {
-          tu = tu + f * (vc - v_env);
-          tv = tv + (-f) * (uc - u_env);
-        }
-        if (dmp) {
-          tu = tu + dmp_u[o];
-          tv = tv + dmp_v[o];
-        }
-        if (heat) tt = tt + (float)s.heat_r[col] * heatz;
-        if (OUTMODE == 0) {
-          uo[o] = uc + dts * tu;
-          vo[o] = vc + dts * tv;
-          tho[o] = thc + dts * tt;
+        cp_async(d, u + ch * nz + k, sizeof(T));
+        cp_async(d + PL, v + ch * nz + k, sizeof(T));
+        cp_async(d + 2 * PL, th + ch * nz + k, sizeof(T));
+      }
+      if (win_) cp_async(d + 3 * PL, w + ch * nzw + k, sizeof(T));
+    }
+    if (kld) cp_async(P + kat, kptr + (ii * ny + jk) * klv + kk, sizeof(T));
+    cp_commit();
+  };
+  // prefill the windows with x = i0-H .. i0+H-1
+  T qu[WIN], qv[WIN], qt[WIN], qw[WIN];
+#pragma unroll
+  for (int r = 1; r < WIN; ++r) {
+    int ii = i0 - H - 1 + r;
+    ii += (ii < 0) ? nx : 0;
+    ii -= (ii >= nx) ? nx : 0;
+    const int c = ii * ny + j;
+    qu[r] = kin ? u[c * nz + k] : (T)0;
+    qv[r] = kin ? v[c * nz + k] : (T)0;
+    qt[r] = kin ? th[c * nz + k] : (T)0;
+    qw[r] = win_ ? w[c * nzw + k] : (T)0;
+  }
+  load_column(i0);
+  copy_halo(i0, plane[0]);
+#pragma unroll 2
+  for (int step = 0; step < nstep; ++step) {
+    const int i = i0 + step;
+#pragma unroll
+    for (int r = 0; r < WIN - 1; ++r) {
+      qu[r] = qu[r + 1];
+      qv[r] = qv[r + 1];
+      qt[r] = qt[r + 1];
+      qw[r] = qw[r + 1];
+    }
+    qu[WIN - 1] = nu;
+    qv[WIN - 1] = nv;
+    qt[WIN - 1] = nt;
+    qw[WIN - 1] = nw;
+    // this step's plane: own row from the window centres (the lid w at level
+    // nz included, where the last chunk has a thread for it; else it is a
+    // level halo), beside the halos copied one step ahead
+    T* P = plane[step & 1];
+    const int pc = (row + H) * kXwCols + lane + 1;
+    if (mine) {
+      P[pc] = qu[H];
+      P[PL + pc] = qv[H];
+      P[2 * PL + pc] = qt[H];
+      P[3 * PL + pc] = qw[H];
+    }
+    if (step + 1 < nstep) load_column(i + 1);
+    cp_wait<0>();
+    __syncthreads();
+    // every thread has left the other plane: its step is the previous one
+    if (step + 1 < nstep) copy_halo(i + 1, plane[(step + 1) & 1]);
+    if (kin && jin) {
+      const T* Pu = P + pc;
+      const T* Pv = Pu + PL;
+      const T* Pt = Pv + PL;
+      const T* Pw = Pt + PL;
+      const int col = i * ny + j;
+      const int o = col * nz + k;
+      const int ow = col * nzw + k;
+      const T uc = qu[H], vc = qv[H], thc = qt[H];
+      T tu = (T)0, tv = (T)0, tt = (T)0;
+      if (adv) {
+        const T wc = (T)0.5 * (qw[H] + Pw[1]);
+        T czu, czv, czt;
+        if (k == 0) {
+          czu = (Pu[1] - uc) * invdz;
+          czv = (Pv[1] - vc) * invdz;
+          czt = (Pt[1] - thc) * invdz;
+        } else if (k == nz - 1) {
+          czu = (uc - Pu[-1]) * invdz;
+          czv = (vc - Pv[-1]) * invdz;
+          czt = (thc - Pt[-1]) * invdz;
         } else {
-          uo[o] = tu;
-          vo[o] = tv;
-          tho[o] = tt;
+          czu = (Pu[1] - Pu[-1]) * inv2dz;
+          czv = (Pv[1] - Pv[-1]) * inv2dz;
+          czt = (Pt[1] - Pt[-1]) * inv2dz;
         }
-        // w on half level k
-        const float wk = qw[3];
-        float tw = 0.0f;
-        if (adv && k > 0) {
-          const float uh = 0.5f * (Pu[pc - 1] + uc);
-          const float vh = 0.5f * (Pv[pc - 1] + vc);
-          const float czw = (Pw[pc + 1] - Pw[pc - 1]) * inv2dz;
-          float xw, yw;
-          if (ws5) {
-            xw = ws5_win(qw, uh, inv60dx);
-            yw = ws5_col(Pw, r0, c, vh, inv60dy);
-          } else {
-            xw = (qw[4] - qw[2]) * inv2dx;
-            yw = (Pw[pc + kXwCols] - Pw[pc - kXwCols]) * inv2dy;
-          }
-          tw = -(uh * xw + vh * yw + wk * czw);
-        }
-        wo[ow] = OUTMODE == 0 ? wk + dts * tw : tw;
-        if (k == nz - 1) {  // the lid, level nz: no tendency
-          const float wl = Pw[pc + 1];
-          wo[ow + 1] = OUTMODE == 0 ? wl : 0.0f;
-        }
+        const T xt = xw_ddx<H, T>(qt, uc, invx), yt = xw_ddy<H, T>(Pt, vc, invy);
+        const T xu = xw_ddx<H, T>(qu, uc, invx), yu = xw_ddy<H, T>(Pu, vc, invy);
+        const T xv = xw_ddx<H, T>(qv, uc, invx), yv = xw_ddy<H, T>(Pv, vc, invy);
+        tt = -(uc * xt + vc * yt + wc * (czt + dth0k));
+        tu = -(uc * xu + vc * yu + wc * czu);
+        tv = -(uc * xv + vc * yv + wc * czv);
+      }
+      if (cor) {
+        tu = tu + f * (vc - (T)s.v_env);
+        tv = tv + (-f) * (uc - (T)s.u_env);
+      }
+      if (drg) {
+        const T up0 = u[col * nz] - (T)s.drag_u_env, vp0 = v[col * nz] - (T)s.drag_v_env;
+        const T ss = up0 * up0 + vp0 * vp0;
+        // above the boundary layer the weight is zero and the root of no use
+        // (0 times the square is 0 or NaN where 0 times the root is)
+        const T al = dragw != (T)0 ? (T)s.drag_rate * sqrt(ss) * dragw : ss * dragw;
+        tu = tu + (-al) * (uc - (T)s.drag_u_env);
+        tv = tv + (-al) * (vc - (T)s.drag_v_env);
+      }
+      if (spg) {
+        tu = tu + (-spa) * (uc - (T)s.sp_u_env);
+        tv = tv + (-spa) * (vc - (T)s.sp_v_env);
+        tt = tt + (-spa) * thc;
+      }
+      if (dif == 1) {
+        const T nu_ = (T)s.diff_nu, rx = (T)s.diff_rdx2, ry = (T)s.diff_rdy2;
+        tu = tu + nu_ * ((qu[H + 1] - (T)2 * uc + qu[H - 1]) * rx +
+                         (Pu[kXwCols] - (T)2 * uc + Pu[-kXwCols]) * ry);
+        tv = tv + nu_ * ((qv[H + 1] - (T)2 * vc + qv[H - 1]) * rx +
+                         (Pv[kXwCols] - (T)2 * vc + Pv[-kXwCols]) * ry);
+      } else if (dif == 2) {
+        const int im = i > 0 ? i - 1 : nx - 1, ip = i + 1 < nx ? i + 1 : 0;
+        const int ox[4] = {0, 0, (im - i) * ny * nz, (ip - i) * ny * nz};
+        const int oy[4] = {0, 0, (jm - j) * nz, (jp - j) * nz};
+        const T nu_ = (T)s.diff_nu, rx = (T)s.diff_rdx2, ry = (T)s.diff_rdy2;
+        tu = tu + (-nu_) * lap5<T, T>(lu, o, ox, oy, rx, ry);
+        tv = tv + (-nu_) * lap5<T, T>(lv, o, ox, oy, rx, ry);
+      }
+      if (col_) tt = tt + (-(T)s.cool_alpha) * thc;
+      if (dmp) {
+        tu = tu + dmp_u[o];
+        tv = tv + dmp_v[o];
+      }
+      if (heat) tt = tt + (T)s.heat_r[col] * heatz;
+      if (OUTMODE == 0) {
+        uo[o] = uc + dts * tu;
+        vo[o] = vc + dts * tv;
+        tho[o] = thc + dts * tt;
+      } else {
+        uo[o] = tu;
+        vo[o] = tv;
+        tho[o] = tt;
+      }
+      // w on half level k
+      const T wk = qw[H];
+      T tw = (T)0;
+      if (adv && k > 0) {
+        const T uh = (T)0.5 * (Pu[-1] + uc);
+        const T vh = (T)0.5 * (Pv[-1] + vc);
+        const T czw = (Pw[1] - Pw[-1]) * inv2dz;
+        const T xw = xw_ddx<H, T>(qw, uh, invx), yw = xw_ddy<H, T>(Pw, vh, invy);
+        tw = -(uh * xw + vh * yw + wk * czw);
+      }
+      if (spg) tw = tw + (-spah) * wk;
+      wo[ow] = OUTMODE == 0 ? wk + dts * tw : tw;
+      if (k == nz - 1) {  // the lid, level nz: no advection
+        const T wl = Pw[1];
+        const T tl = spg ? (-(T)s.sp_ah[nz]) * wl : (T)0;
+        wo[ow + 1] = OUTMODE == 0 ? wl + dts * tl : tl;
       }
     }
-    __syncthreads();  // the next chunk's first step rewrites plane 0
   }
 }
 
