@@ -241,6 +241,11 @@ int oracle_b200_step(OraclePlan *plan, const OracleStatePtrs *in, const OracleSt
  * compatibility and discrete residuals of this solve. */
 int oracle_b200_project(OraclePlan *plan, void *u, void *v, void *w, void *phi,
                         int log_diag, void *stream);
+/* The same from (u, v, w) into (uo, vo, wo): each output is its own input or
+ * overlaps none of the fields. */
+int oracle_b200_project_to(OraclePlan *plan, const void *u, const void *v, const void *w,
+                           void *uo, void *vo, void *wo, void *phi, int log_diag,
+                           void *stream);
 
 /* anelastic_divergence (tendency.py:393-437): d = div(rho u). */
 int oracle_b200_divergence(OraclePlan *plan, const void *u, const void *v, const void *w,

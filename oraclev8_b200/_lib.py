@@ -26,7 +26,7 @@ LIB_PATH = Path(__file__).resolve().parent / "liboracle_b200.so"
 
 EXPORTS = (
     "oracle_b200_plan_create", "oracle_b200_plan_destroy", "oracle_b200_plan_scratch_bytes",
-    "oracle_b200_step", "oracle_b200_project", "oracle_b200_divergence",
+    "oracle_b200_step", "oracle_b200_project", "oracle_b200_project_to", "oracle_b200_divergence",
     "oracle_b200_phi_gradient", "oracle_b200_poisson_solve", "oracle_b200_apply_operator",
     "oracle_b200_buoyancy", "oracle_b200_tendency", "oracle_b200_read_diag",
     "oracle_b200_last_error", "oracle_b200_version", "oracle_b200_launch_count",
@@ -114,6 +114,7 @@ def load(path: Path | None = None):
         "oracle_b200_plan_scratch_bytes": ([vp], c_size_t),
         "oracle_b200_step": ([vp, POINTER(StatePtrs), POINTER(StatePtrs), c_double, c_int, vp], c_int),
         "oracle_b200_project": ([vp, vp, vp, vp, vp, c_int, vp], c_int),
+        "oracle_b200_project_to": ([vp] * 8 + [c_int, vp], c_int),
         "oracle_b200_divergence": ([vp, vp, vp, vp, vp, vp], c_int),
         "oracle_b200_phi_gradient": ([vp, vp, vp, vp, vp, vp], c_int),
         "oracle_b200_poisson_solve": ([vp, vp, vp, c_int, vp], c_int),

@@ -258,6 +258,13 @@ class Plan:
                                              self._ptr(w, self.wshape), self._ptr(phi, s),
                                              int(log_diag), self._stream()))
 
+    def project_to(self, u, v, w, uo, vo, wo, phi, log_diag=False):
+        s, ws = self.shape, self.wshape
+        L.check(self.lib.oracle_b200_project_to(
+            self.handle, self._ptr(u, s), self._ptr(v, s), self._ptr(w, ws), self._ptr(uo, s),
+            self._ptr(vo, s), self._ptr(wo, ws), self._ptr(phi, s), int(log_diag),
+            self._stream()))
+
     def divergence(self, u, v, w, out=None):
         out = self.empty() if out is None else out
         s = self.shape

@@ -3320,22 +3320,29 @@ int oracle_b200_step_graph_destroy(OracleStepGraph* g) {
   return OB_OK;
 }
 
-int oracle_b200_project(OraclePlan* p, void* u, void* v, void* w, void* phi, int log_diag,
-                        void* stream) {
+int oracle_b200_project_to(OraclePlan* p, const void* u, const void* v, const void* w, void* uo,
+                           void* vo, void* wo, void* phi, int log_diag, void* stream) {
   if (int rc = check_plan(p)) return rc;
-  if (!u || !v || !w || !phi) return fail(OB_ERR_ARG, "project: NULL pointer");
+  if (!u || !v || !w || !uo || !vo || !wo || !phi)
+    return fail(OB_ERR_ARG, "project: NULL pointer");
   cudaStream_t st = (cudaStream_t)stream;
   const int de = p->diag_every;
   if (log_diag) p->diag_every = 1;
   int rc = DISPATCH(p,
-                    project_impl<double>(p, (double*)u, (double*)v, (double*)w, nullptr, -1.0,
-                                         (double*)u, (double*)v, (double*)w, (double*)phi,
-                                         OB_DIAG_LAST_COMPAT, OB_DIAG_LAST_DISC, st),
-                    project_impl<float>(p, (float*)u, (float*)v, (float*)w, nullptr, -1.0,
-                                        (float*)u, (float*)v, (float*)w, (float*)phi,
-                                        OB_DIAG_LAST_COMPAT, OB_DIAG_LAST_DISC, st));
+                    project_impl<double>(p, (const double*)u, (const double*)v, (const double*)w,
+                                         nullptr, -1.0, (double*)uo, (double*)vo, (double*)wo,
+                                         (double*)phi, OB_DIAG_LAST_COMPAT, OB_DIAG_LAST_DISC,
+                                         st),
+                    project_impl<float>(p, (const float*)u, (const float*)v, (const float*)w,
+                                        nullptr, -1.0, (float*)uo, (float*)vo, (float*)wo,
+                                        (float*)phi, OB_DIAG_LAST_COMPAT, OB_DIAG_LAST_DISC, st));
   p->diag_every = de;
   return rc;
+}
+
+int oracle_b200_project(OraclePlan* p, void* u, void* v, void* w, void* phi, int log_diag,
+                        void* stream) {
+  return oracle_b200_project_to(p, u, v, w, u, v, w, phi, log_diag, stream);
 }
 
 int oracle_b200_divergence(OraclePlan* p, const void* u, const void* v, const void* w, void* d,
