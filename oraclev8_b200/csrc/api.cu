@@ -1,4 +1,5 @@
 // C ABI of the B200 LH82 step library.  See include/oracle_b200.h.
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -1737,15 +1738,25 @@ void slow_xw_launch(OraclePlan* p, int mask, double dts, const T* u, const T* v,
                     const T* th, T* uo, T* vo, T* wo, T* tho, cudaStream_t st) {
   const int nx = p->g.nx, nk = (p->g.nz + 31) / 32, kw = (p->g.nz + nk - 1) / nk;
   const int nrow = (p->g.ny + kXwTJ - 1) / kXwTJ;
-  int dev = 0, nsm = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  // segments: four CTAs per SM where the grid gives them, 7 to 35 columns
-  // (each segment loads its window's 2 H columns again)
-  const int want = std::max(1, 4 * nsm / (nrow * nk));
-  const int seg = std::min(35, std::max(7, ((nx + want - 1) / want + 6) / 7 * 7));
-  const dim3 grid(nrow, (nx + seg - 1) / seg, nk);
   const int threads = std::max(128, (kXwTJ * kw + 31) / 32 * 32);
+  // The segments' number: fewest column steps over whole waves of resident CTAs.
+  // A segment also costs its window's first columns, about H + 2 steps.  (Four
+  // CTAs per SM and at most 35 columns left the last wave nearly empty: a step of
+  // 320 x 320 x 32 production FP64 1366 -> 1314 us, the advection of
+  // 360 x 300 x 60 FP32 127 -> 121 us.)
+  const int res = resident_ctas(k_slow_xw<T, OUT, H, PROD>, threads, 0);
+  int seg = nx;
+  long best = LONG_MAX;
+  for (int n = 1; n <= std::max(1, nx / 7); ++n) {
+    const int sg = (nx + n - 1) / n;
+    const long ctas = (long)nrow * nk * ((nx + sg - 1) / sg);
+    const long cost = (ctas + res - 1) / res * (sg + H + 2);
+    if (cost < best) {
+      best = cost;
+      seg = sg;
+    }
+  }
+  const dim3 grid(nrow, (nx + seg - 1) / seg, nk);
   k_slow_xw<T, OUT, H, PROD><<<grid, threads, 0, st>>>(p->g, slow_args(p), mask, dts, seg, kw, u,
                                                        v, w, th, (const T*)p->Du,
                                                        (const T*)p->Dv, uo, vo, wo, tho);
