@@ -1273,8 +1273,9 @@ __global__ void __launch_bounds__(256, PROD ? 5 : 4) k_slow_f32(GridK g, SlowK s
 // suffices.  H = 3: WS5 advection; H = 1: centred or none.
 // What bounds it: the gather forms wait on ~48 loads a cell, whose x and y
 // neighbours other CTAs own too; this one loads about 7 and waits on the
-// arithmetic and the shared-memory reads of the y stencils (24 a cell) at the
-// 16 (double) or 24 warps per SM its windows leave.  Two steps a turn of the
+// shared-memory reads of the y and z neighbours (28 a cell: the first-level
+// cache's pipe was 77 to 81% busy, DRAM 23 to 48%, with 32) at the 16 (double) or
+// 24 warps per SM its windows leave.  Two steps a turn of the
 // loop halve the moves of the window's rotation (seven, which would make it a
 // renaming, spill in double precision).  Same terms and order as the gather
 // forms.  Gather against march, a slow half (us): 512 x 512 x 64 double, WS5,
@@ -1285,7 +1286,8 @@ __global__ void __launch_bounds__(256, PROD ? 5 : 4) k_slow_f32(GridK g, SlowK s
 constexpr int kXwTJ = 8;         // rows per CTA
 constexpr int kXwCols = 32 + 2;  // plane columns: k0-1 .. k0+32
 
-// values at offsets -3 .. 3 of q (window) or of column c (plane, row stride kXwCols)
+// values at offsets -3 .. 3: a window's, or a plane column's about q (row stride
+// kXwCols) whose own value q0 is in a register
 template <class T>
 __device__ __forceinline__ T ws5_win(const T (&q)[7], T a, T inv60d) {
   const bool up = a >= (T)0;
@@ -1295,10 +1297,10 @@ __device__ __forceinline__ T ws5_win(const T (&q)[7], T a, T inv60d) {
   return (up ? d : -d) * inv60d;
 }
 template <class T>
-__device__ __forceinline__ T ws5_col(const T* q, T a, T inv60d) {
+__device__ __forceinline__ T ws5_col(const T* q, T q0, T a, T inv60d) {
   const bool up = a >= (T)0;
   const int s = up ? kXwCols : -kXwCols;
-  const T d = (T)-2 * q[-3 * s] + (T)15 * q[-2 * s] - (T)60 * q[-s] + (T)20 * q[0] +
+  const T d = (T)-2 * q[-3 * s] + (T)15 * q[-2 * s] - (T)60 * q[-s] + (T)20 * q0 +
               (T)30 * q[s] - (T)3 * q[2 * s];
   return (up ? d : -d) * inv60d;
 }
@@ -1309,8 +1311,8 @@ __device__ __forceinline__ T xw_ddx(const T (&q)[2 * H + 1], T a, T inv) {
   else return (q[2] - q[0]) * inv;
 }
 template <int H, class T>
-__device__ __forceinline__ T xw_ddy(const T* q, T a, T inv) {
-  if constexpr (H == 3) return ws5_col<T>(q, a, inv);
+__device__ __forceinline__ T xw_ddy(const T* q, T q0, T a, T inv) {
+  if constexpr (H == 3) return ws5_col<T>(q, q0, a, inv);
   else return (q[kXwCols] - q[-kXwCols]) * inv;
 }
 
@@ -1475,9 +1477,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3) k_slow_xw(
           czv = (Pv[1] - Pv[-1]) * inv2dz;
           czt = (Pt[1] - Pt[-1]) * inv2dz;
         }
-        const T xt = xw_ddx<H, T>(qt, uc, invx), yt = xw_ddy<H, T>(Pt, vc, invy);
-        const T xu = xw_ddx<H, T>(qu, uc, invx), yu = xw_ddy<H, T>(Pu, vc, invy);
-        const T xv = xw_ddx<H, T>(qv, uc, invx), yv = xw_ddy<H, T>(Pv, vc, invy);
+        const T xt = xw_ddx<H, T>(qt, uc, invx), yt = xw_ddy<H, T>(Pt, thc, vc, invy);
+        const T xu = xw_ddx<H, T>(qu, uc, invx), yu = xw_ddy<H, T>(Pu, uc, vc, invy);
+        const T xv = xw_ddx<H, T>(qv, uc, invx), yv = xw_ddy<H, T>(Pv, vc, vc, invy);
         tt = -(uc * xt + vc * yt + wc * (czt + dth0k));
         tu = -(uc * xu + vc * yu + wc * czu);
         tv = -(uc * xv + vc * yv + wc * czv);
@@ -1536,7 +1538,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3) k_slow_xw(
         const T uh = (T)0.5 * (Pu[-1] + uc);
         const T vh = (T)0.5 * (Pv[-1] + vc);
         const T czw = (Pw[1] - Pw[-1]) * inv2dz;
-        const T xw = xw_ddx<H, T>(qw, uh, invx), yw = xw_ddy<H, T>(Pw, vh, invy);
+        const T xw = xw_ddx<H, T>(qw, uh, invx), yw = xw_ddy<H, T>(Pw, wk, vh, invy);
         tw = -(uh * xw + vh * yw + wk * czw);
       }
       if (spg) tw = tw + (-spah) * wk;
