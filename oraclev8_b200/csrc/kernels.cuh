@@ -1280,7 +1280,7 @@ __global__ void __launch_bounds__(256, PROD ? 5 : 4) k_slow_f32(GridK g, SlowK s
 // renaming, spill in double precision).  Same terms and order as the gather
 // forms.  Gather against march, a slow half (us): 512 x 512 x 64 double, WS5,
 // 640 -> 405; 320 x 320 x 32 double, production, 198 -> 115; 360 x 300 x 60
-// single, WS5, 133 -> 119.
+// single, WS5, 133 -> 115.
 // grid = (ceil(ny / 8), ceil(nx / seg), ceil(nz / kw)); block: at least
 // max(8 kw, 128) threads.
 constexpr int kXwTJ = 8;         // rows per CTA
