@@ -288,8 +288,8 @@ __device__ __forceinline__ void z_last_inv(const ZPlan& p, const cplx<T>* buf, i
 }
 
 // ---- level pairs -----------------------------------------------------------------
-// Two adjacent levels of one field at element index i (the first level's);
-// vec: the pair is aligned (an even level count); nb: the second level exists.
+// Two adjacent levels of one field, the first at p; vec: one access for both, which
+// wants p on a multiple of its size (zpairs); two: the second level exists.
 template <class TS>
 struct __align__(2 * sizeof(TS)) pair2 {
   TS a, b;
@@ -487,11 +487,12 @@ __device__ __forceinline__ void z_last_bfly(const ZPlan& p, const cplx<T>* line,
 }
 
 // Forward x transforms; RL: the line's last radix (a switch over it here costs
-// the compiler the registers).  grid = (ceil(nz / levels), ceil(ny / RY)); dynamic
+// the compiler the registers); fvec: the fields' level pairs (zpairs), apart from
+// the spectra's, which lie in the plan's own buffers.  grid = (ceil(nz / levels), ceil(ny / RY)); dynamic
 // shared memory: RY lines.
 template <class T, class TS, int MODE, int RL>
 __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
-    const __grid_constant__ ZPlan p, GridK g, int RY, const TS* __restrict__ u,
+    const __grid_constant__ ZPlan p, GridK g, int RY, bool fvec, const TS* __restrict__ u,
     const TS* __restrict__ v, const TS* __restrict__ w, const TS* __restrict__ bh, double sdt,
     const double* __restrict__ rho, const double* __restrict__ rhoh, const T* __restrict__ kx,
     const cplx<T>* __restrict__ tw, cplx<T>* __restrict__ X0, cplx<T>* __restrict__ X1,
@@ -528,7 +529,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
       const TS* q = f + (n * ny + y0 + row) * nz + z;
       pair2<TS> a[R];
 #pragma unroll
-      for (int j = 0; j < R; ++j) a[j] = ldpair(q + j * step * xs, vec, two);
+      for (int j = 0; j < R; ++j) a[j] = ldpair(q + j * step * xs, fvec, two);
 #pragma unroll
       for (int j = 0; j < R; ++j)
         r[j] = weigh ? mk<T>(wmul(ra, (T)a[j].a), wmul(rb, (T)a[j].b))
@@ -619,7 +620,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
 //    2 C levels, 2 C - 1 interfaces.
 template <class T, class TS, int MODE, int RL>
 __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
-    const __grid_constant__ ZPlan p, GridK g, int RY, const cplx<T>* __restrict__ S1,
+    const __grid_constant__ ZPlan p, GridK g, int RY, bool fvec, const cplx<T>* __restrict__ S1,
     const cplx<T>* __restrict__ S2, const T* __restrict__ kx, const cplx<T>* __restrict__ tw,
     const TS* u_in, const TS* v_in, const TS* w_in, const TS* __restrict__ bh, double sdt,
     TS* u_out, TS* v_out, TS* w_out, TS* phi_out) {
@@ -741,7 +742,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
         pair2<TS> a[R];
         if (MODE != ZIX_FIELDS && MODE != ZIX_GRAD) {
 #pragma unroll
-          for (int j = 0; j < R; ++j) a[j] = ldpair(in + o + j * step * xs, vec, two);
+          for (int j = 0; j < R; ++j) a[j] = ldpair(in + o + j * step * xs, fvec, two);
         }
         cplx<T> x[R];
 #pragma unroll
@@ -754,7 +755,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
             r0 = (TS)((T)a[j].a - x[j].x);
             r1 = (TS)((T)a[j].b - x[j].y);
           }
-          stpair(out + o + j * step * xs, r0, r1, vec, two);
+          stpair(out + o + j * step * xs, r0, r1, fvec, two);
         }
       });
       return;

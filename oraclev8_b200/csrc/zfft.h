@@ -1,6 +1,8 @@
 // Host interface of the level-paired line transforms (zfft.cuh): line plans and
 // launchers, compiled apart from the C ABI (zfft.cu, once per precision).
 #pragma once
+#include <cstdint>
+
 #include "common.cuh"
 
 namespace ob {
@@ -25,6 +27,16 @@ bool zplan_make(int N, int elem, ZPlan* out);
 
 // The index into W_N^t of every entry of the line's pass twiddles (N entries).
 void zplan_twiddles(const ZPlan& p, int* t);
+
+// Whether the level pairs of a call's fields move as one access each: an even level
+// count, so that every column starts on a pair, and every field on a multiple of the
+// pair's size.  A caller's field need not: a view into a larger buffer starts on any
+// element, and goes level by level.
+template <class TS, class... P>
+inline bool zpairs(int nz, const P*... fields) {
+  return !(nz & 1) &&
+         (... && (reinterpret_cast<std::uintptr_t>(fields) % (2 * sizeof(TS)) == 0));
+}
 
 // One direction's lines: plan and device tables.
 template <class T>
