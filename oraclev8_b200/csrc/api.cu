@@ -253,7 +253,8 @@ struct OraclePlan {
   int refine_passes = 0, refine_every = 1;
   long step_count = 0;
   int capturing = 0;  // recording a step graph: no solver-residual logging
-  unsigned logged = 0;  // diag slots that hold a logged solve's residuals
+  unsigned logged = 0;           // diag slots that hold a logged solve's residuals
+  unsigned logged_recorded = 0;  // slots that a graph of the caller's may fill at any time
   size_t esz = 8;  // element size of T
   // device constants
   double *kx = nullptr, *ky = nullptr, *rho = nullptr, *rhoh = nullptr, *theta0 = nullptr;
@@ -1323,6 +1324,32 @@ int proj_ix(OraclePlan* p, bool stage, const T* u, const T* v, const T* w, const
   return OB_OK;
 }
 
+// The residual slots of a solve, before it runs: cleared unless it logs, in which
+// case it writes them.  They are zero until a solve logs, so clearing is left out
+// where none has since the last time (two clears a projection took 15 us of a
+// step's 400 at 96 x 96 x 32).  What a caller records into a graph of their own
+// runs at any later time, any number of times: recorded clears are never left out,
+// and after a recorded solve that logs none is.  A step graph's steps do not log
+// and clear their slots in one go (step_impl).
+int residual_slots(OraclePlan* p, bool log, int slot_c, int slot_d, cudaStream_t st) {
+  if (p->capturing) return OB_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  OB_CUDA(cudaStreamIsCapturing(st, &cap));
+  const bool recorded = cap != cudaStreamCaptureStatusNone;
+  const unsigned bits = (1u << slot_c) | (1u << slot_d);
+  if (log) {  // the sum of squares is accumulated
+    OB_CUDA(cudaMemsetAsync(p->diag + slot_d, 0, sizeof(double), st));
+    (recorded ? p->logged_recorded : p->logged) |= bits;
+    return OB_OK;
+  }
+  if (recorded || ((p->logged | p->logged_recorded) & bits)) {
+    OB_CUDA(cudaMemsetAsync(p->diag + slot_c, 0, sizeof(double), st));
+    OB_CUDA(cudaMemsetAsync(p->diag + slot_d, 0, sizeof(double), st));
+  }
+  if (!recorded) p->logged &= ~bits;
+  return OB_OK;
+}
+
 // stage_sdt < 0: in-place projection of (u, v, w) with phi output.
 // stage_sdt >= 0: inputs are the anchor state (u, v, w, th); the provisional
 // stage state w + sdt * b_half is formed on the fly and the projected result
@@ -1342,26 +1369,8 @@ int project_impl(OraclePlan* p, const T* u, const T* v, const T* w, const T* th,
   p->solve_count += 1;
   const int de = p->diag_every < 1 ? 1 : p->diag_every;
   const bool log = !p->capturing && ((de == 1) || (p->solve_count % de == 1));
-  double* diag = nullptr;
-  // The residual slots of a solve that does not log read zero.  They are zero
-  // until one logs, so only its traces are cleared: at once in recorded work,
-  // which may run after one that logged (a step clears all its own in one go),
-  // and else where one did.  Two clears a projection took 15 us of a step's 400
-  // at 96 x 96 x 32.
-  const unsigned bits = (1u << slot_c) | (1u << slot_d);
-  if (log) {
-    diag = p->diag;
-    OB_CUDA(cudaMemsetAsync(p->diag + slot_d, 0, sizeof(double), st));
-    p->logged |= bits;
-  } else if (!p->capturing) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    OB_CUDA(cudaStreamIsCapturing(st, &cap));
-    if ((p->logged & bits) || cap != cudaStreamCaptureStatusNone) {
-      OB_CUDA(cudaMemsetAsync(p->diag + slot_c, 0, sizeof(double), st));
-      OB_CUDA(cudaMemsetAsync(p->diag + slot_d, 0, sizeof(double), st));
-    }
-    if (cap == cudaStreamCaptureStatusNone) p->logged &= ~bits;
-  }
+  RC(residual_slots(p, log, slot_c, slot_d, st));
+  double* diag = log ? p->diag : nullptr;
   const bool stage = stage_sdt >= 0.0;
   if (shared && sizeof(T) == 4 && stage) {
     { Launch L_(p, 1, st); fy4sh(p, (float)stage_sdt, st); }
@@ -2110,7 +2119,7 @@ int solve_impl(OraclePlan* p, const T* d, T* phi, int log_diag, cudaStream_t st)
   double* diag = nullptr;
   if (log_diag) {
     diag = p->diag;
-    OB_CUDA(cudaMemsetAsync(p->diag + OB_DIAG_LAST_DISC, 0, sizeof(double), st));
+    RC(residual_slots(p, true, OB_DIAG_LAST_COMPAT, OB_DIAG_LAST_DISC, st));
   }
   const long ncols = (long)g.nxh * g.ny;
   { Launch L_(p, 2, st); k_thomas<T, kThomasCols><<<(unsigned)((ncols + kThomasCols - 1) / kThomasCols), kThomasCols,
