@@ -1870,9 +1870,13 @@ int step_impl(OraclePlan* p, const OracleStatePtrs* in, const OracleStatePtrs* o
                    p->diffusion;
   const int all = OB_TEND_ADVECTION | OB_TEND_CORIOLIS | OB_TEND_DAMPING | OB_TEND_HEATING |
                   OB_TEND_DRAG | OB_TEND_SPONGE | OB_TEND_DIFFUSION | OB_TEND_COOLING;
-  if (p->capturing)
-    OB_CUDA(cudaMemsetAsync(p->diag + OB_DIAG_COMPAT0, 0,
-                            (OB_DIAG_LAST_DISC + 1 - OB_DIAG_COMPAT0) * sizeof(double), st));
+  // recorded steps do not log: the slots of their solves read zero, the others stay
+  if (p->capturing && p->projection) {
+    if (p->buoyancy)
+      OB_CUDA(cudaMemsetAsync(p->diag + OB_DIAG_COMPAT0, 0, 6 * sizeof(double), st));
+    if (mom || !p->buoyancy)
+      OB_CUDA(cudaMemsetAsync(p->diag + OB_DIAG_LAST_COMPAT, 0, 2 * sizeof(double), st));
+  }
   // anchor state y^n after the first slow half step
   const T *au = (const T*)in->u, *av = (const T*)in->v, *aw = (const T*)in->w,
           *ath = (const T*)in->theta_prime, *aphi = (const T*)in->phi;

@@ -9,7 +9,7 @@ from tests.gpu_helpers import dev
 
 pytestmark = pytest.mark.gpu
 
-LAST = slice(12, 14)  # include/oracle_b200.h, OB_DIAG_*
+STAGES, LAST = slice(6, 12), slice(12, 14)  # include/oracle_b200.h, OB_DIAG_*
 
 
 def _plan(prec, nx=48, ny=40, nz=9, **kw):
@@ -73,3 +73,20 @@ def test_an_unlogged_projection_clears_what_a_replayed_graph_logged(prec):
             assert not p.read_diag()[LAST].any()
     del logs, quiet
     torch.cuda.synchronize()
+
+
+def test_a_step_graph_clears_the_slots_of_its_own_solves_only():
+    # buoyancy and projection alone: a step solves in its three stages, not for the state itself
+    p = _plan("fp64", buoyancy=True, poisson_diag_every=1)
+    u, v, w = _fields(p)
+    s = [u, v, w, torch.ones_like(u), torch.zeros_like(u)]
+    ptr = p.state_ptrs(*s)
+    p.project(u, v, w, s[4], log_diag=True)
+    p.step(ptr, ptr, 1.0, True)
+    before = p.read_diag()
+    assert before[LAST].any() and before[STAGES].any()
+    g = p.step_graph(ptr, 1.0, 1)
+    g.launch()
+    after = p.read_diag()
+    assert not after[STAGES].any()
+    np.testing.assert_array_equal(after[LAST], before[LAST])
