@@ -1137,26 +1137,6 @@ int make_zsolve(OraclePlan* p) {
   return OB_OK;
 }
 
-// The residuals of a solve that logs them, where its solution comes from the
-// plane form: the generic sweeps in place on S3, whose result nothing reads.
-template <class T>
-int thomas_residuals(OraclePlan* p, double* diag, int slot_c, int slot_d, cudaStream_t st) {
-  const long ncols = (long)p->g.nxh * p->g.ny;
-  const unsigned nb = (unsigned)((ncols + kThomasCols - 1) / kThomasCols);
-  cplx<T>* S3 = (cplx<T>*)p->S3;
-  if (sizeof(T) == 8 || !p->lw_blocks) {
-    { Launch L_(p, 2, st); k_thomas<T, kThomasCols><<<nb, kThomasCols, smem_thomas(p), st>>>(
-          p->g, thomas_args(p), S3, S3, diag, slot_c, slot_d); }
-  } else {
-    { Launch L_(p, 2, st); k_thomas<T, kThomasCols, double><<<(unsigned)p->n_lw, kThomasCols, smem_thomas(p, 8), st>>>(
-          p->g, thomas_args(p), S3, S3, diag, slot_c, slot_d, p->lw_blocks, nullptr); }
-    { Launch L_(p, 2, st); k_thomas<T, kThomasCols, float><<<nb, kThomasCols, smem_thomas(p, 4), st>>>(
-          p->g, thomas_args(p), S3, S3, diag, slot_c, slot_d, nullptr, p->lw_flag); }
-  }
-  OB_LAUNCHED();
-  return OB_OK;
-}
-
 // ---- projection pipeline -------------------------------------------------
 // One launcher per kernel class of the projection; each runs the variant the
 // plan's choice fields select (register-resident > compile-time-chunk pencils
@@ -1269,13 +1249,14 @@ int proj_iy(OraclePlan* p, int cls, cudaStream_t st) {
 }
 
 // the plane form: forward y of (X0, X1) (or their spectrum itself), the solve
-// and inverse y into (S1, out1), in place
+// and inverse y into (S1, out1), in place; diag: logs this solve's residuals (fwd
+// only: S3, no input of it, keeps the source meanwhile)
 template <class T>
 int proj_yz(OraclePlan* p, int cls, bool fwd, const cplx<T>* X0, const cplx<T>* X1, cplx<T>* out1,
-            cudaStream_t st) {
+            cudaStream_t st, double* diag = nullptr, int slot_c = 0, int slot_d = 0) {
   Launch L_(p, cls, st);
   OB_CUDA(zplane<T>(zline_y<T>(p), p->g, thomas_args(p), zsolve_args(p), fwd, X0, X1,
-                    (cplx<T>*)p->S1, out1, st));
+                    (cplx<T>*)p->S1, out1, ZLog<T>{diag, slot_c, slot_d, (cplx<T>*)p->S3}, st));
   return OB_OK;
 }
 
@@ -1378,11 +1359,8 @@ int project_impl(OraclePlan* p, const T* u, const T* v, const T* w, const T* th,
   } else {
     RC(proj_fx<T>(p, stage, u, v, w, th, bh, stage_sdt, st));
     if (p->z_yz) {
-      if (diag) {
-        RC(proj_fy<T>(p, st));
-        RC(thomas_residuals<T>(p, diag, slot_c, slot_d, st));
-      }
-      RC(proj_yz<T>(p, 2, true, (cplx<T>*)p->S1, (cplx<T>*)p->S2, (cplx<T>*)p->S2, st));
+      RC(proj_yz<T>(p, 2, true, (cplx<T>*)p->S1, (cplx<T>*)p->S2, (cplx<T>*)p->S2, st, diag,
+                    slot_c, slot_d));
       return proj_ix<T>(p, stage, u, v, w, th, bh, stage_sdt, uo, vo, wo, phio, st);
     }
     RC(proj_fy<T>(p, st));
@@ -2114,17 +2092,18 @@ template <class T>
 int solve_impl(OraclePlan* p, const T* d, T* phi, int log_diag, cudaStream_t st) {
   using C = cplx<T>;
   const GridK g = p->g;
-  if (sizeof(T) == 8 && p->z_yz && !log_diag) {  // FP32 plans solve every column in double here
-    RC(fwd_x<T>(p, d, st));
-    RC(proj_yz<T>(p, 2, true, (C*)p->S1, nullptr, nullptr, st));
-    return op_ix_field<T>(p, phi, st);
-  }
-  RC(fwd_scalar<T>(p, d, st));
   double* diag = nullptr;
   if (log_diag) {
     diag = p->diag;
     RC(residual_slots(p, true, OB_DIAG_LAST_COMPAT, OB_DIAG_LAST_DISC, st));
   }
+  if (sizeof(T) == 8 && p->z_yz) {  // FP32 plans solve every column in double here
+    RC(fwd_x<T>(p, d, st));
+    RC(proj_yz<T>(p, 2, true, (C*)p->S1, nullptr, nullptr, st, diag, OB_DIAG_LAST_COMPAT,
+                  OB_DIAG_LAST_DISC));
+    return op_ix_field<T>(p, phi, st);
+  }
+  RC(fwd_scalar<T>(p, d, st));
   const long ncols = (long)g.nxh * g.ny;
   { Launch L_(p, 2, st); k_thomas<T, kThomasCols><<<(unsigned)((ncols + kThomasCols - 1) / kThomasCols), kThomasCols,
                              smem_thomas(p), st>>>(g, thomas_args(p), (C*)p->S3, (C*)p->S3,

@@ -185,7 +185,8 @@ cudaError_t zfft_init<T>() {
   OB_Z(attr(k_zfy2<T, T, ZFY_HELM, C / 2>));
   OB_Z(attr(k_ziy<T, true>));
   OB_Z(attr(k_ziy<T, false>));
-  OB_Z(attr(k_zplane<T>));
+  OB_Z(attr(k_zplane<T, false>));
+  OB_Z(attr(k_zplane<T, true>));
 #if OB_ZWIDE
   OB_Z(attr(k_zfy2<T, float, ZFY_RESID, C>));
   OB_Z(attr(k_zfy2<T, float, ZFY_RESID, C / 2>));
@@ -289,7 +290,7 @@ int zplane_group<T>(const ZPlan& p, int nz) {
 template <>
 cudaError_t zplane<T>(const ZLine<T>& l, const GridK& g, const ThomasK& t, const ZSolve& s,
                       bool fwd, const cplx<T>* X0, const cplx<T>* X1, cplx<T>* out0, cplx<T>* out1,
-                      cudaStream_t st) {
+                      const ZLog<T>& log, cudaStream_t st) {
   const int group = zplane_group<T>(l.plan, g.nz);
   if (!group) return cudaErrorInvalidValue;
   const size_t smem = zplane_layout<T>(l.plan.NP, g.nz, group).total;
@@ -297,8 +298,13 @@ cudaError_t zplane<T>(const ZLine<T>& l, const GridK& g, const ThomasK& t, const
   // a warp more than the columns fill, for the zero mode, where that costs none
   const int threads = std::min(kZPlaneThreads,
                                std::max({128, div_up(per, 64) * 64, div_up(g.ny, 32) * 32 + 32}));
-  k_zplane<T><<<g.nxh, threads, smem, st>>>(l.plan, g, group, fwd, X0, X1, l.k, l.tw, t, s.inv,
-                                            s.dpd, s.lw, out0, out1);
+  if (log.diag && !fwd) return cudaErrorInvalidValue;
+  if (log.diag)
+    k_zplane<T, true><<<g.nxh, threads, smem, st>>>(l.plan, g, group, fwd, X0, X1, l.k, l.tw, t,
+                                                    s.inv, s.dpd, s.lw, out0, out1, log);
+  else
+    k_zplane<T, false><<<g.nxh, threads, smem, st>>>(l.plan, g, group, fwd, X0, X1, l.k, l.tw, t,
+                                                     s.inv, s.dpd, s.lw, out0, out1, log);
   return cudaGetLastError();
 }
 

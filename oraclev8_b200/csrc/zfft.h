@@ -92,13 +92,20 @@ struct ZSolve {
   cplx<double>* dpd;          // scratch of that shape, single precision only
   const unsigned char* lw;    // per 32 columns: long waves (single precision)
 };
+// Where a solve logs its residuals; diag null: it does not.
+template <class T>
+struct ZLog {
+  double* diag;
+  int slot_c, slot_d;   // compatibility residual; sum of |L phi^ - d^|^2, added to
+  cplx<T>* src;         // scratch of the source's size, (nx / 2 + 1, ny, nz)
+};
 // level chunks per group of the plane's scratch; 0: the plane does not fit
 template <class T>
 int zplane_group(const ZPlan& p, int nz);
 template <class T>
 cudaError_t zplane(const ZLine<T>& l, const GridK& g, const ThomasK& t, const ZSolve& s,
                    bool fwd, const cplx<T>* X0, const cplx<T>* X1, cplx<T>* out0, cplx<T>* out1,
-                   cudaStream_t st);
+                   const ZLog<T>& log, cudaStream_t st);
 cudaError_t zplane_inv(const GridK& g, const ThomasK& t, double* inv, cudaStream_t st);
 
 }  // namespace ob

@@ -45,19 +45,28 @@ static __global__ void k_zinv(GridK g, ThomasK t, double* __restrict__ inv) {
 // pivots at inv[k ny]; DP: the eliminated values wait for the way back in dp,
 // else in the column, rounded to T.  Pivots (and dp on the way back) are loaded a
 // batch ahead of the chain that uses them; first: the pivots of levels
-// 0 .. kZBatch - 1, loaded before the block's barrier.
+// 0 .. kZBatch - 1, loaded before the block's barrier.  LOG: returns the sum of
+// |L phi^ - d^|^2 over the levels (poisson.py:263-268), of the column's solution
+// as it is found (DP and double: before its last rounding) and its source in r.
 constexpr int kZBatch = 8;
+// One column's source, as the plane's solve found it, and what L needs of it.
+template <class T>
+struct ZResid {
+  const cplx<T>* d;    // nz levels
+  const double *rho, *rhoh;
+  double ksq, dz2;
+};
 __device__ __forceinline__ void z_pivots(double* v, const double* __restrict__ inv, int k0,
                                          int nz, int ny) {
 #pragma unroll
   for (int j = 0; j < kZBatch; ++j)
     v[j] = (k0 + j >= 0 && k0 + j < nz) ? __ldg(inv + (size_t)(k0 + j) * ny) : 0.0;
 }
-template <class T, bool DP>
-__device__ __forceinline__ void z_sweep(cplx<T>* col, int nz, int ny,
-                                        const double* __restrict__ inv, const double* a,
-                                        const double* c, double scale, cplx<double>* dp,
-                                        const double* first) {
+template <class T, bool DP, bool LOG>
+__device__ __forceinline__ double z_sweep(cplx<T>* col, int nz, int ny,
+                                          const double* __restrict__ inv, const double* a,
+                                          const double* c, double scale, cplx<double>* dp,
+                                          const double* first, const ZResid<T>& r) {
   double cur[kZBatch], nxt[kZBatch];
   double pr = 0.0, pi = 0.0;
 #pragma unroll
@@ -80,6 +89,20 @@ __device__ __forceinline__ void z_sweep(cplx<T>* col, int nz, int ny,
     }
   }
   col[nz - 1] = mk<T>((T)(pr * scale), (T)(pi * scale));
+  // residual: the level above and the flux through its top
+  double acc = 0.0, ur = 0.0, ui = 0.0, fr = 0.0, fi = 0.0;
+  auto as_found = [](double x) { return DP ? x : (double)(T)x; };
+  auto row = [&](int k, double fur, double fui, double flr, double fli) {  // level k, (ur, ui)
+    const cplx<T> d = r.d[k];
+    const double q = r.ksq * r.rho[k];
+    const double rr = (fur - flr) / r.dz2 - q * ur - (double)d.x;
+    const double ri = (fui - fli) / r.dz2 - q * ui - (double)d.y;
+    acc += rr * rr + ri * ri;
+  };
+  if (LOG) {
+    ur = as_found(pr);
+    ui = as_found(pi);
+  }
   // batches downward from level nz - 2: levels k0 .. k0 - kZBatch + 1
   cplx<double> dc[DP ? kZBatch : 1], dn[DP ? kZBatch : 1];
   auto values = [&](int k0) {
@@ -111,15 +134,29 @@ __device__ __forceinline__ void z_sweep(cplx<T>* col, int nz, int ny,
       pr = srn(d.x, mrn(cp, pr));
       pi = srn(d.y, mrn(cp, pi));
       col[k] = mk<T>((T)(pr * scale), (T)(pi * scale));
+      if (LOG) {
+        const double xr = as_found(pr), xi = as_found(pi);
+        const double flr = r.rhoh[k + 1] * (ur - xr), fli = r.rhoh[k + 1] * (ui - xi);
+        row(k + 1, fr, fi, flr, fli);
+        fr = flr;
+        fi = fli;
+        ur = xr;
+        ui = xi;
+      }
     }
   }
+  if (LOG) row(0, fr, fi, 0.0, 0.0);
+  return acc;
 }
 
 // The zero mode (poisson.py:256, 316-325, 367-383) of one column, in double: the
 // mean removed, the reduced system with phi(0, 0, 0) = 0.  w: 5 nz doubles, the
-// last 3 nz the reduced system's a0, cp0, inv0.
-template <class T>
-__device__ void z_zero_mode(cplx<T>* col, int nz, double scale, double* w) {
+// last 3 nz the reduced system's a0, cp0, inv0.  LOG: returns the residual against
+// the whole source less its mean (the zero mode of a real field is real), and the
+// compatibility residual (poisson.py:233-236) in *compat.
+template <class T, bool LOG>
+__device__ double z_zero_mode(cplx<T>* col, int nz, double scale, double* w, const ZResid<T>& r,
+                              double dz, double* compat) {
   const double *a0 = w + 2 * nz, *cp0 = w + 3 * nz, *inv0 = w + 4 * nz;
   double sr = 0, si = 0;
 #pragma unroll 4
@@ -127,6 +164,7 @@ __device__ void z_zero_mode(cplx<T>* col, int nz, double scale, double* w) {
     sr = arn(sr, (double)col[k].x);
     si = arn(si, (double)col[k].y);
   }
+  if (LOG) *compat = hypot(mrn(sr, dz), mrn(si, dz));
   const double mr = drn(sr, (double)nz), mi = drn(si, (double)nz);
   double pr = 0, pi = 0;
 #pragma unroll 4
@@ -139,12 +177,27 @@ __device__ void z_zero_mode(cplx<T>* col, int nz, double scale, double* w) {
   }
   col[0] = mk<T>((T)0, (T)0);
   col[nz - 1] = mk<T>((T)(pr * scale), (T)(pi * scale));
+  double above = pr, fu = 0.0, s1 = 0.0, s2 = 0.0;
+  auto row = [&](int k, double fl) {  // of level k: its value above, the flux fl below it
+    const double q = (fu - fl) / r.dz2 - (double)r.d[k].x;
+    s1 += q;
+    s2 += q * q;
+    fu = fl;
+  };
 #pragma unroll 4
   for (int j = nz - 3; j >= 0; --j) {
     pr = srn(w[2 * j], mrn(cp0[j], pr));
     pi = srn(w[2 * j + 1], mrn(cp0[j], pi));
     col[j + 1] = mk<T>((T)(pr * scale), (T)(pi * scale));
+    if (LOG) {
+      row(j + 2, r.rhoh[j + 2] * (above - pr));
+      above = pr;
+    }
   }
+  if (!LOG) return 0.0;
+  row(1, r.rhoh[1] * above);
+  row(0, 0.0);
+  return s2 - s1 * s1 / nz;
 }
 
 constexpr int kZPlaneThreads = 512;
@@ -176,13 +229,15 @@ __host__ __device__ inline ZPlaneLayout zplane_layout(int NP, int nz, int group)
 // null: phi~ alone.  The outputs may be the inputs (a block reads its plane before
 // it writes).  inv: reciprocal pivots.  Single precision: the columns of a block
 // of 32 that lw flags (nearly singular, long waves) keep their eliminated values
-// in double, in dpd.
-template <class T>
+// in double, in dpd.  LOG (with fwd): the residuals of this solution into log, the
+// source kept in log.src until the sweep returns to it; the solution is the one an
+// unlogged solve gives.
+template <class T, bool LOG>
 __global__ void __launch_bounds__(kZPlaneThreads, 1) k_zplane(
     const __grid_constant__ ZPlan p, GridK g, int group, int fwd, const cplx<T>* X0,
     const cplx<T>* X1, const T* __restrict__ ky, const cplx<T>* __restrict__ tw,
     const __grid_constant__ ThomasK t, const double* __restrict__ inv, cplx<double>* dpd,
-    const unsigned char* __restrict__ lw, cplx<T>* out0, cplx<T>* out1) {
+    const unsigned char* __restrict__ lw, cplx<T>* out0, cplx<T>* out1, ZLog<T> log) {
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   constexpr int C = zy_cols<T>();
   constexpr int LC = zlog2(C);
@@ -286,6 +341,12 @@ __global__ void __launch_bounds__(kZPlaneThreads, 1) k_zplane(
           cplx<T>* q = line + zphys(p, b) * st;
 #pragma unroll
           for (int j = 0; j < R; ++j) q[j * Qp] = f[j];
+          if (LOG) {
+            const int z = (c0 + row) * C + c;
+#pragma unroll
+            for (int j = 0; j < R; ++j)
+              if (z < nz) log.src[(kx * ny + b + p.Q * j) * nz + z] = f[j];
+          }
         }
       });
     }
@@ -296,6 +357,16 @@ __global__ void __launch_bounds__(kZPlaneThreads, 1) k_zplane(
   double first[kZBatch];
   if (threadIdx.x < ny) z_pivots(first, inv + plane + threadIdx.x, 0, nz, ny);
   __syncthreads();
+  double resid = 0.0, compat = 0.0;
+  auto source = [&](int k) {
+    ZResid<T> r{};
+    if (LOG) {
+      const double a = t.kx[kx], b = t.ky[k];
+      r = {log.src + (size_t)(kx * ny + k) * nz, t.rho, t.rhoh, arn(mrn(a, a), mrn(b, b)),
+           t.dz * t.dz};
+    }
+    return r;
+  };
 #pragma unroll 1
   for (int k = threadIdx.x; k < ny; k += blockDim.x) {
     if (kx == 0 && k == 0) continue;
@@ -303,11 +374,21 @@ __global__ void __launch_bounds__(kZPlaneThreads, 1) k_zplane(
     const size_t at = plane + k;
     if (k != threadIdx.x) z_pivots(first, inv + at, 0, nz, ny);
     if (sizeof(T) == 4 && lw[(kx * ny + k) >> 5])
-      z_sweep<T, true>(col, nz, ny, inv + at, ad, cd, t.scale, dpd + at, first);
+      resid += z_sweep<T, true, LOG>(col, nz, ny, inv + at, ad, cd, t.scale, dpd + at, first,
+                                     source(k));
     else
-      z_sweep<T, false>(col, nz, ny, inv + at, ad, cd, t.scale, nullptr, first);
+      resid += z_sweep<T, false, LOG>(col, nz, ny, inv + at, ad, cd, t.scale, nullptr, first,
+                                      source(k));
   }
-  if (kx == 0 && threadIdx.x == ((blockDim.x - 1) & ~31)) z_zero_mode<T>(pl, nz, t.scale, zw);
+  if (LOG && kx && 2 * kx != g.nx) resid *= 2.0;  // the half spectrum's other half
+  if (kx == 0 && threadIdx.x == ((blockDim.x - 1) & ~31)) {
+    resid += z_zero_mode<T, LOG>(pl, nz, t.scale, zw, source(0), t.dz, &compat);
+    if (LOG) log.diag[log.slot_c] = compat;
+  }
+  if (LOG) {
+    for (int o = 16; o > 0; o >>= 1) resid += __shfl_xor_sync(0xffffffffu, resid, o);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&log.diag[log.slot_d], resid);
+  }
   __syncthreads();
 
   // inverse lines: i ky' phi^ through the scratch (by groups), phi^ in the plane
