@@ -3221,7 +3221,13 @@ int oracle_b200_plan_create(const OracleGridDesc* grid, const OracleComponentDes
   if (p->prec == OB_PREC_F32 && (rc = make_refiner(p, kx.data(), ky.data()))) return bail(rc);
   if ((rc = p->prec == OB_PREC_F64 ? make_zsolve<double>(p) : make_zsolve<float>(p)))
     return bail(rc);
-  p->z_yz = p->zinv != nullptr;
+  // untimed, the plane form only where every plane has an SM at once: a second wave
+  // leaves most of them idle.  A step, plane form / separate launches (us):
+  // within one wave 192 x 192 x 48 double 815 / 829, 256 x 256 x 48 single 983 /
+  // 1109; beyond it 320 x 320 x 32 double 1700 / 1344, 1000 x 300 x 40 double
+  // 5883 / 5501, 384 x 384 x 48 single 2098 / 1950 (1000 x 300 x 40 single, four
+  // short waves, 3826 / 3898: left to the autotuner, which times both)
+  p->z_yz = p->zinv && p->g.nxh <= nsm;
   // allocations and table copies complete: the memory is usable on any stream
   if (cudaStreamSynchronize(p->astream) != cudaSuccess)
     return bail(fail(OB_ERR_CUDA, "plan_create: set-up stream failed"));

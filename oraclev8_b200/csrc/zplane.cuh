@@ -15,8 +15,8 @@
 // launches against this one (us): 128 x 128 x 32 double 44.6 -> 27; 96 x 96 x 32
 // single 48 -> 23, 250 x 162 x 45 single 70 -> 39 (with the long waves' double
 // sweep, which the separate solve runs beside the others).  Planes that need a
-// second wave of blocks lose: 320 x 320 x 32 double 91 -> 157; the autotuner
-// times both.
+// second wave of blocks mostly lose: 320 x 320 x 32 double 91 -> 157.  A plan that
+// is not tuned takes this form for grids of one wave; the autotuner times both.
 #pragma once
 #include "zfft.cuh"
 
