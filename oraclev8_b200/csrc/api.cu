@@ -23,6 +23,7 @@
 #include "vdiag.cuh"
 #include "init.cuh"
 #include "zfft.h"
+#include "resident.h"
 
 using namespace ob;
 
@@ -929,33 +930,25 @@ void fx4(const OraclePlan* q, int zc, const float* u, const float* v, const floa
     }
   }
 }
-// Resident CTAs of a persistent kernel on the current device (occupancy API x
-// SM count), cached per (kernel, device): kernels of one signature share a
-// function-pointer type, so the cache is keyed by the pointer itself.
-std::mutex g_resident_mu;
-std::map<std::pair<const void*, int>, int> g_resident;
+// Resident CTAs of a kernel on the current device (occupancy API x SM count) at
+// this block size and shared memory, cached.
+ResidentCache g_resident;
 
 template <class K>
 int resident_ctas(K kernel, int threads, size_t smem) {
   int dev = 0;
   cudaGetDevice(&dev);
-  const auto key = std::make_pair(reinterpret_cast<const void*>(kernel), dev);
-  {
-    std::lock_guard<std::mutex> lk(g_resident_mu);
-    auto it = g_resident.find(key);
-    if (it != g_resident.end()) return it->second;
-  }
-  int nsm = 148, per = 1;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) != cudaSuccess ||
-      per < 1) {
-    cudaGetLastError();
-    per = 1;
-  }
-  const int n = per * nsm;
-  std::lock_guard<std::mutex> lk(g_resident_mu);
-  g_resident[key] = n;
-  return n;
+  return g_resident.get(reinterpret_cast<const void*>(kernel), dev, threads, smem, [&] {
+    int nsm = 148, per = 1;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) !=
+            cudaSuccess ||
+        per < 1) {
+      cudaGetLastError();
+      per = 1;
+    }
+    return per * nsm;
+  });
 }
 
 template <int MODE, int ZC>
