@@ -270,7 +270,7 @@ struct OraclePlan {
   void *S4 = nullptr, *S5 = nullptr, *S6 = nullptr;
   void *Au = nullptr, *Av = nullptr, *Aw = nullptr, *Ath = nullptr, *Aphi = nullptr;
   void *Su = nullptr, *Sv = nullptr, *Sw = nullptr, *Sphi = nullptr;
-  void *Du = nullptr, *Dv = nullptr;                         // damper / temp
+  void *Du = nullptr, *Dv = nullptr;  // the damper's tendency (Dv with damping only); Du temporary
   void* Bh = nullptr;  // half-level buoyancy of the step's anchor theta' (nz + 1 levels)
   double* diag = nullptr;
   DiagPart* parts = nullptr;
@@ -2322,7 +2322,7 @@ int tune_impl(OraclePlan* p, cudaStream_t st) {
   const size_t e = p->esz;
   // finite inputs: zero every buffer a candidate reads
   for (void* b : {p->Au, p->Av, p->Ath, p->Aphi, p->Su, p->Sv, p->Sphi, p->Du, p->Dv})
-    OB_CUDA(cudaMemsetAsync(b, 0, n * e, st));
+    if (b) OB_CUDA(cudaMemsetAsync(b, 0, n * e, st));
   for (void* b : {p->Aw, p->Sw}) OB_CUDA(cudaMemsetAsync(b, 0, nw * e, st));
   if (p->Bh) OB_CUDA(cudaMemsetAsync(p->Bh, 0, nw * e, st));
   const T *u = (const T*)p->Au, *v = (const T*)p->Av, *w = (const T*)p->Aw,
@@ -3154,7 +3154,7 @@ int oracle_b200_plan_create(const OracleGridDesc* grid, const OracleComponentDes
       (rc = dalloc(p, &p->Ath, n * e)) || (rc = dalloc(p, &p->Aphi, n * e)) ||
       (rc = dalloc(p, &p->Su, n * e)) || (rc = dalloc(p, &p->Sv, n * e)) ||
       (rc = dalloc(p, &p->Sw, nw * e)) || (rc = dalloc(p, &p->Sphi, n * e)) ||
-      (rc = dalloc(p, &p->Du, n * e)) || (rc = dalloc(p, &p->Dv, n * e)))
+      (rc = dalloc(p, &p->Du, n * e)) || (p->damping && (rc = dalloc(p, &p->Dv, n * e))))
     return bail(rc);
   if (p->diffusion == OB_DIFF_BIHARMONIC &&
       ((rc = dalloc(p, &p->Lu, n * e)) || (rc = dalloc(p, &p->Lv, n * e))))

@@ -167,7 +167,10 @@ def build_run(req: RunRequest, device_dtype=None, blowup_u_max: float = BLOWUP_U
 def footprint_bytes(req: RunRequest) -> int:
     """HBM a resident run holds: 5 state fields and the plan's scratch (3
     half-spectrum buffers, 5 anchor and 4 stage fields, 2 temporaries and the
-    half-level buoyancy; plus two FP64 spectra for the FP32-refined
+    half-level buoyancy; the reciprocal pivots of the plane form, 8 (n / 2 + 1) n nz
+    bytes where a plane fits shared memory, are there instead of the second
+    temporary, which only the damper has, and of the production physics' unused
+    buoyancy; plus two FP64 spectra for the FP32-refined
     correction; the production physics adds the damper's two tendency fields
     and the biharmonic's two inner Laplacians; single-precision 1024 x 1024
     runs with fast stages add the three spectra of the shared stage
