@@ -103,10 +103,10 @@ cudaError_t zfx_last(int mode, const ZLine<T>& l, const GridK& g, const TS* u, c
   constexpr int C = zx_pairs<T>();
   const int sets = mode == ZFX_FIELDS && !v ? 1 : mode == ZFX_SHARED ? 3 : 2;
   const Shape s = shape<T>(l.plan, C, 1, g.ny, sets * div_up(g.nz, 2 * C), zx_threads<T>());
-  const bool fvec = zpairs<TS>(g.nz, u, v);
+  const bool pairs = zpairs<TS>(g.nz, u, v);
 #define OB_ZFX(M)                                                                              \
   case M:                                                                                      \
-    k_zfx<T, TS, M, RL><<<s.grid, s.threads, s.smem, st>>>(l.plan, g, s.rows, fvec, u, v, w, bh, \
+    k_zfx<T, TS, M, RL><<<s.grid, s.threads, s.smem, st>>>(l.plan, g, s.rows, pairs, u, v, w, bh, \
                                                            sdt, rho, rhoh, l.k, l.tw, X0, X1,  \
                                                            X2);                                \
     break;
@@ -135,10 +135,10 @@ cudaError_t zix_last(int mode, const ZLine<T>& l, const GridK& g, const cplx<T>*
                      : mode != ZIX_GRAD && phio ? 2 * chunks + div_up(g.nz, 2 * C - 1)
                                                 : 3 * chunks;
   const Shape s = shape<T>(l.plan, C, 1, g.ny, blocks, zx_threads<T>());
-  const bool fvec = zpairs<T>(g.nz, u, v, uo, vo);
+  const bool pairs = zpairs<T>(g.nz, u, v, uo, vo);
 #define OB_ZIX(M)                                                                               \
   case M:                                                                                       \
-    k_zix<T, T, M, RL><<<s.grid, s.threads, s.smem, st>>>(l.plan, g, s.rows, fvec, S1, S2, l.k, \
+    k_zix<T, T, M, RL><<<s.grid, s.threads, s.smem, st>>>(l.plan, g, s.rows, pairs, S1, S2, l.k, \
                                                           l.tw, u, v, w, bh, sdt, uo, vo, wo,   \
                                                           phio);                                \
     break;

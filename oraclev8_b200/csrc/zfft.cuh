@@ -487,12 +487,11 @@ __device__ __forceinline__ void z_last_bfly(const ZPlan& p, const cplx<T>* line,
 }
 
 // Forward x transforms; RL: the line's last radix (a switch over it here costs
-// the compiler the registers); fvec: the fields' level pairs (zpairs), apart from
-// the spectra's, which lie in the plan's own buffers.  grid = (ceil(nz / levels), ceil(ny / RY)); dynamic
-// shared memory: RY lines.
+// the compiler the registers); pairs: level pairs in one access each (zpairs).
+// grid = (ceil(nz / levels), ceil(ny / RY)); dynamic shared memory: RY lines.
 template <class T, class TS, int MODE, int RL>
 __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
-    const __grid_constant__ ZPlan p, GridK g, int RY, bool fvec, const TS* __restrict__ u,
+    const __grid_constant__ ZPlan p, GridK g, int RY, bool pairs, const TS* __restrict__ u,
     const TS* __restrict__ v, const TS* __restrict__ w, const TS* __restrict__ bh, double sdt,
     const double* __restrict__ rho, const double* __restrict__ rhoh, const T* __restrict__ kx,
     const cplx<T>* __restrict__ tw, cplx<T>* __restrict__ X0, cplx<T>* __restrict__ X1,
@@ -508,7 +507,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
   const int sets = MODE == ZFX_FIELDS && !v ? 1 : SETS;
   const int chunk = blockIdx.x / sets, set = blockIdx.x - chunk * sets;
   const int z = (chunk * C + (threadIdx.x & (C - 1))) * 2;  // the thread's first level
-  const bool on = z < nz, two = z + 1 < nz, vec = !(nz & 1);
+  const bool on = z < nz, two = z + 1 < nz, vec = pairs;
   const int rows = min(RY, ny - y0);
   const int xs = ny * nz, ws = ny * (nz + 1);
   zwt<T> ra{}, rb{}, f0{}, f1{}, f2{};
@@ -529,7 +528,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
       const TS* q = f + (n * ny + y0 + row) * nz + z;
       pair2<TS> a[R];
 #pragma unroll
-      for (int j = 0; j < R; ++j) a[j] = ldpair(q + j * step * xs, fvec, two);
+      for (int j = 0; j < R; ++j) a[j] = ldpair(q + j * step * xs, vec, two);
 #pragma unroll
       for (int j = 0; j < R; ++j)
         r[j] = weigh ? mk<T>(wmul(ra, (T)a[j].a), wmul(rb, (T)a[j].b))
@@ -620,7 +619,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
 //    2 C levels, 2 C - 1 interfaces.
 template <class T, class TS, int MODE, int RL>
 __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
-    const __grid_constant__ ZPlan p, GridK g, int RY, bool fvec, const cplx<T>* __restrict__ S1,
+    const __grid_constant__ ZPlan p, GridK g, int RY, bool pairs, const cplx<T>* __restrict__ S1,
     const cplx<T>* __restrict__ S2, const T* __restrict__ kx, const cplx<T>* __restrict__ tw,
     const TS* u_in, const TS* v_in, const TS* w_in, const TS* __restrict__ bh, double sdt,
     TS* u_out, TS* v_out, TS* w_out, TS* phi_out) {
@@ -643,7 +642,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
   const int c = threadIdx.x & (C - 1);
   const int z = pot ? chunk * (2 * C - 1) - 1 + 2 * c : (chunk * C + c) * 2;
   const bool on = z < nz, two = z + 1 < nz, one = z >= 0;
-  const bool vec = !(nz & 1) && !pot;
+  const bool vec = pairs && !pot;
   const int rows = min(RY, ny - y0);
   const int xs = ny * nz, ws = ny * (nz + 1);
   const T idz = (T)(1.0 / g.dz);
@@ -742,7 +741,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
         pair2<TS> a[R];
         if (MODE != ZIX_FIELDS && MODE != ZIX_GRAD) {
 #pragma unroll
-          for (int j = 0; j < R; ++j) a[j] = ldpair(in + o + j * step * xs, fvec, two);
+          for (int j = 0; j < R; ++j) a[j] = ldpair(in + o + j * step * xs, vec, two);
         }
         cplx<T> x[R];
 #pragma unroll
@@ -755,7 +754,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
             r0 = (TS)((T)a[j].a - x[j].x);
             r1 = (TS)((T)a[j].b - x[j].y);
           }
-          stpair(out + o + j * step * xs, r0, r1, fvec, two);
+          stpair(out + o + j * step * xs, r0, r1, vec, two);
         }
       });
       return;
