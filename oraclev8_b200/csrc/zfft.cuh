@@ -383,11 +383,46 @@ __device__ __forceinline__ T wdiff(zwt<T> ru, T wu, zwt<T> rl, T wl) {
     return srn(mrn(ru.h, wu), mrn(rl.h, wl));
   }
 }
+// the same of values with what their own rounding left, which counts where they
+// nearly cancel
+template <class T>
+struct zval {
+  T h, l;
+};
+template <class T>
+__device__ __forceinline__ T wdiff(zwt<T> ru, zval<T> wu, zwt<T> rl, zval<T> wl) {
+  if constexpr (sizeof(T) == 4) {
+    const float q = wl.h * rl.h;
+    const float e = fmaf(-wl.h, rl.h, q);
+    const float r = fmaf(wu.h, ru.h, -q);
+    const float t = fmaf(wu.l, ru.h, -(wl.l * rl.h));
+    return r + (e + fmaf(wu.h, ru.l, fmaf(-wl.h, rl.l, t)));
+  } else {
+    return wdiff(ru, wu.h, rl, wl.h);
+  }
+}
 
-// provisional stage w: w + sdt b (integrator.py:483-490), rounded once in
-// single precision
-__device__ __forceinline__ double zstage(double w, double sdt, double b) { return arn(w, mrn(sdt, b)); }
-__device__ __forceinline__ float zstage(float w, float sdt, float b) { return fmaf(sdt, b, w); }
+// Provisional stage w: w + sdt b (integrator.py:483-490).  Single precision: the
+// sum in two floats, so that the flux difference of its values is as good as in
+// double.  Rounded to one float first, it would add an ulp of w over dz to the
+// source, more than all its other roundings where w is large against sdt b.
+__device__ __forceinline__ zval<double> zstage(double w, zwt<double> sdt, double b) {
+  return {arn(w, mrn(sdt.h, b)), 0.0};
+}
+__device__ __forceinline__ zval<float> zstage(float w, zwt<float> sdt, float b) {
+  const float p = mrn(sdt.h, b);
+  const float e = fmaf(sdt.l, b, fmaf(sdt.h, b, -p));  // sdt b - p
+  const float s = arn(w, p);
+  const float x = srn(s, w);                           // the part of p that s took
+  return {s, arn(arn(srn(w, srn(s, x)), srn(p, x)), e)};
+}
+// the same rounded once (an infinite sum has no remainder)
+template <class T>
+__device__ __forceinline__ T zstage1(T w, zwt<T> sdt, T b) {
+  const zval<T> s = zstage(w, sdt, b);
+  if (sizeof(T) == 8 || isnan(s.l)) return s.h;
+  return s.h + s.l;
+}
 
 // Level pairs per CTA.  A warp's access costs the first-level cache one pass
 // per 128-byte line it touches, and these kernels are bound by those passes
@@ -519,7 +554,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
     f1 = mkwt<T>(rhoh[z + 1] * id);
     f2 = mkwt<T>(two ? rhoh[z + 2] * id : 0.0);
   }
-  const T sd = (T)sdt;
+  const zwt<T> sd = mkwt<T>(sdt);
   // rows of a field at this thread's level pair, weighted
   auto field = [&](const TS* f, bool weigh) {
     return [=](auto rc, int row, int c, int n, int step, cplx<T>* r) {
@@ -549,18 +584,17 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
         w1[j] = (T)q[1];
         w2[j] = two ? (T)q[2] : (T)0;
       }
-      if (MODE == ZFX_STAGE) {
 #pragma unroll
-        for (int j = 0; j < R; ++j) {
+      for (int j = 0; j < R; ++j) {
+        if (MODE == ZFX_STAGE) {
           const TS* q = b + o + j * step * ws;
-          w0[j] = zstage(w0[j], sd, (T)q[0]);
-          w1[j] = zstage(w1[j], sd, (T)q[1]);
-          if (two) w2[j] = zstage(w2[j], sd, (T)q[2]);
+          const zval<T> s0 = zstage(w0[j], sd, (T)q[0]), s1 = zstage(w1[j], sd, (T)q[1]);
+          const zval<T> s2 = zstage(w2[j], sd, two ? (T)q[2] : (T)0);
+          r[j] = mk<T>(wdiff(f1, s1, f0, s0), two ? wdiff(f2, s2, f1, s1) : (T)0);
+        } else {
+          r[j] = mk<T>(wdiff(f1, w1[j], f0, w0[j]), two ? wdiff(f2, w2[j], f1, w1[j]) : (T)0);
         }
       }
-#pragma unroll
-      for (int j = 0; j < R; ++j)
-        r[j] = mk<T>(wdiff(f1, w1[j], f0, w0[j]), two ? wdiff(f2, w2[j], f1, w1[j]) : (T)0);
     };
   };
   // A set's lines in turn: rho u (X0 = i kx' times it), then D w, added to X0: the
@@ -646,7 +680,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
   const int rows = min(RY, ny - y0);
   const int xs = ny * nz, ws = ny * (nz + 1);
   const T idz = (T)(1.0 / g.dz);
-  const T sd = (T)sdt;
+  const zwt<T> sd = mkwt<T>(sdt);
 
     const cplx<T>* src = run == 1 ? S2 : S1;
     const bool gx = MODE != ZIX_FIELDS && run == 0;
@@ -782,8 +816,8 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
 #pragma unroll
           for (int j = 0; j < R; ++j) {
             const TS* t = bh + wo + j * step * ws;
-            if (la) a[j] = (TS)zstage((T)a[j], sd, (T)t[0]);
-            if (lb) b[j] = (TS)zstage((T)b[j], sd, (T)t[1]);
+            if (la) a[j] = (TS)zstage1<T>((T)a[j], sd, (T)t[0]);
+            if (lb) b[j] = (TS)zstage1<T>((T)b[j], sd, (T)t[1]);
           }
         }
         cplx<T> x[R];
@@ -809,7 +843,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
           for (int j = 0; j < R; ++j) {
             const int top = wo + j * step * ws + (nz - z);
             TS t = w_in[top];
-            if (MODE == ZIX_STAGE) t = (TS)zstage((T)t, sd, (T)bh[top]);
+            if (MODE == ZIX_STAGE) t = (TS)zstage1<T>((T)t, sd, (T)bh[top]);
             w_out[top] = t;
           }
         }
@@ -831,8 +865,8 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
 #pragma unroll
           for (int j = 0; j < R; ++j) {
             const TS* q = bh + o + j * step * ws;
-            a[j] = (TS)zstage((T)a[j], sd, (T)q[0]);
-            b[j] = (TS)zstage((T)b[j], sd, (T)q[1]);
+            a[j] = (TS)zstage1<T>((T)a[j], sd, (T)q[0]);
+            b[j] = (TS)zstage1<T>((T)b[j], sd, (T)q[1]);
           }
         }
       }
@@ -857,7 +891,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
         for (int j = 0; j < R; ++j) {
           const int top = o + j * step * ws + (two ? 2 : 1);
           TS t = w_in[top];
-          if (MODE == ZIX_STAGE) t = (TS)zstage((T)t, sd, (T)bh[top]);
+          if (MODE == ZIX_STAGE) t = (TS)zstage1<T>((T)t, sd, (T)bh[top]);
           w_out[top] = t;
         }
       }
