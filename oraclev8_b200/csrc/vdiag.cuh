@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kVdThreads) k_vd_speed_max(
     }
     for (long long o = nv * V + first; o < n; o += stride)
       m.take((double)u[o] - ue, (double)v[o] - ve, o);
-  } else if (ncol * band.n < 0x7fffffffLL) {
+  } else if (ncol * band.n < (1LL << 30)) {  // 32 bits, with room for the steps past the end
     const int n = (int)(ncol * band.n);
 #pragma unroll 4
     for (int e = (int)first; e < n; e += (int)stride) {
