@@ -304,7 +304,7 @@ cudaError_t zplane<T>(const ZLine<T>& l, const GridK& g, const ThomasK& t, const
                                                     s.inv, s.dpd, s.lw, out0, out1, log);
   else
     k_zplane<T, false><<<g.nxh, threads, smem, st>>>(l.plan, g, group, fwd, X0, X1, l.k, l.tw, t,
-                                                     s.inv, s.dpd, s.lw, out0, out1, log);
+                                                     s.inv, s.dpd, s.lw, out0, out1, ZNoLog{});
   return cudaGetLastError();
 }
 

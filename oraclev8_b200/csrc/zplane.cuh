@@ -202,6 +202,11 @@ __device__ double z_zero_mode(cplx<T>* col, int nz, double scale, double* w, con
 
 constexpr int kZPlaneThreads = 512;
 
+// a kernel that logs nothing takes no argument for it
+struct ZNoLog {};
+template <class T, bool LOG>
+using ZLogArg = std::conditional_t<LOG, ZLog<T>, ZNoLog>;
+
 // Shared memory of a plane block (bytes from the dynamic base): the plane's
 // slots (every column of a wavenumber, their count made odd so the sweep's
 // lanes fall on distinct banks), the scratch lines of `group` level chunks, the
@@ -237,7 +242,7 @@ __global__ void __launch_bounds__(kZPlaneThreads, 1) k_zplane(
     const __grid_constant__ ZPlan p, GridK g, int group, int fwd, const cplx<T>* X0,
     const cplx<T>* X1, const T* __restrict__ ky, const cplx<T>* __restrict__ tw,
     const __grid_constant__ ThomasK t, const double* __restrict__ inv, cplx<double>* dpd,
-    const unsigned char* __restrict__ lw, cplx<T>* out0, cplx<T>* out1, ZLog<T> log) {
+    const unsigned char* __restrict__ lw, cplx<T>* out0, cplx<T>* out1, ZLogArg<T, LOG> log) {
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   constexpr int C = zy_cols<T>();
   constexpr int LC = zlog2(C);
@@ -341,7 +346,7 @@ __global__ void __launch_bounds__(kZPlaneThreads, 1) k_zplane(
           cplx<T>* q = line + zphys(p, b) * st;
 #pragma unroll
           for (int j = 0; j < R; ++j) q[j * Qp] = f[j];
-          if (LOG) {
+          if constexpr (LOG) {
             const int z = (c0 + row) * C + c;
 #pragma unroll
             for (int j = 0; j < R; ++j)
@@ -360,7 +365,7 @@ __global__ void __launch_bounds__(kZPlaneThreads, 1) k_zplane(
   double resid = 0.0, compat = 0.0;
   auto source = [&](int k) {
     ZResid<T> r{};
-    if (LOG) {
+    if constexpr (LOG) {
       const double a = t.kx[kx], b = t.ky[k];
       r = {log.src + (size_t)(kx * ny + k) * nz, t.rho, t.rhoh, arn(mrn(a, a), mrn(b, b)),
            t.dz * t.dz};
@@ -383,9 +388,9 @@ __global__ void __launch_bounds__(kZPlaneThreads, 1) k_zplane(
   if (LOG && kx && 2 * kx != g.nx) resid *= 2.0;  // the half spectrum's other half
   if (kx == 0 && threadIdx.x == ((blockDim.x - 1) & ~31)) {
     resid += z_zero_mode<T, LOG>(pl, nz, t.scale, zw, source(0), t.dz, &compat);
-    if (LOG) log.diag[log.slot_c] = compat;
+    if constexpr (LOG) log.diag[log.slot_c] = compat;
   }
-  if (LOG) {
+  if constexpr (LOG) {
     for (int o = 16; o > 0; o >>= 1) resid += __shfl_xor_sync(0xffffffffu, resid, o);
     if ((threadIdx.x & 31) == 0) atomicAdd(&log.diag[log.slot_d], resid);
   }
