@@ -1147,7 +1147,7 @@ int proj_fx(OraclePlan* p, bool stage, const T* u, const T* v, const T* w, const
   Launch L_(p, 0, st);
   if (stage ? (bh && p->z_fxs) : p->z_fx) {
     OB_CUDA((zfx<T, T>(stage ? ZFX_STAGE : ZFX_DIV, zline_x<T>(p), g, u, v, w, bh, sdt, p->rho,
-                       p->rhoh, S1, S2, nullptr, st)));
+                       p->rhoh, S1, S2, st)));
     return OB_OK;
   }
   if constexpr (sizeof(T) == 4) {
@@ -1198,8 +1198,7 @@ int proj_fy(OraclePlan* p, cudaStream_t st) {
   C* S3 = (C*)p->S3;
   Launch L_(p, 1, st);
   if (p->z_fy) {
-    OB_CUDA((zfy<T, T>(ZFY_DIV, zline_y<T>(p), g, S1, S2, nullptr, 0.0, p->kx, p->ky, S3,
-                       nullptr, st)));
+    OB_CUDA((zfy<T, T>(ZFY_DIV, zline_y<T>(p), g, S1, S2, 0.0, p->kx, p->ky, S3, nullptr, st)));
     return OB_OK;
   }
   if (sizeof(T) == 4 && p->zc4_fy)
@@ -1382,7 +1381,7 @@ int refine_fx(OraclePlan* p, const float* u, const float* v, const float* w, cud
   Launch L_(p, OB_PROF_REFINE, st);
   if (p->z_fxd) {
     OB_CUDA((zfx<double, float>(ZFX_DIV, zline_x<double>(q), g, u, v, w, nullptr, 0.0, p->rho,
-                                p->rhoh, R1, R2, nullptr, st)));
+                                p->rhoh, R1, R2, st)));
     return OB_OK;
   }
   if (p->zc4_fxd)
@@ -1409,8 +1408,8 @@ int refine_fy(OraclePlan* p, cudaStream_t st) {
   cplx<float>* S3 = (cplx<float>*)p->S3;
   Launch L_(p, OB_PROF_REFINE, st);
   if (p->z_fyd) {
-    OB_CUDA((zfy<double, float>(ZFY_RESID, zline_y<double>(q), g, R1, R2, nullptr, 0.0, q->kx,
-                                q->ky, S3, nullptr, st)));
+    OB_CUDA((zfy<double, float>(ZFY_RESID, zline_y<double>(q), g, R1, R2, 0.0, q->kx, q->ky, S3,
+                                nullptr, st)));
     return OB_OK;
   }
   if (p->zc4_fyd) {
@@ -1520,7 +1519,7 @@ int damper_impl(OraclePlan* p, const T* u, const T* v, double dt_slow, cudaStrea
   C* S2 = (C*)p->S2;
   if (p->z_fx)
     { Launch L_(p, 0, st); OB_CUDA((zfx<T, T>(ZFX_FIELDS, zline_x<T>(p), g, u, v, nullptr, nullptr,
-                                              0.0, p->rho, p->rhoh, S1, S2, nullptr, st))); }
+                                              0.0, p->rho, p->rhoh, S1, S2, st))); }
   else if (sizeof(T) == 4 && p->zc3_fx)
     { Launch L_(p, 0, st); fx3f(p, p->zc3_fx, (const float*)u, (const float*)v, (cplx<float>*)S1,
                                (cplx<float>*)S2, st); }
@@ -1532,8 +1531,7 @@ int damper_impl(OraclePlan* p, const T* u, const T* v, double dt_slow, cudaStrea
   const double scale = -(p->epsilon / dt_slow) / ((double)g.nx * (double)g.ny);
   if (p->z_fy) {
     Launch L_(p, 1, st);
-    OB_CUDA((zfy<T, T>(ZFY_HELM, zline_y<T>(p), g, S1, S2, nullptr, scale, p->kx, p->ky, S1, S2,
-                       st)));
+    OB_CUDA((zfy<T, T>(ZFY_HELM, zline_y<T>(p), g, S1, S2, scale, p->kx, p->ky, S1, S2, st)));
   } else if (sizeof(T) == 4 && p->zc3_fy) {
     // forward y, multipliers and inverse y in one register-resident pass
     { Launch L_(p, 1, st); hy(p, scale, (cplx<float>*)S1, (cplx<float>*)S2, st); }
@@ -1966,7 +1964,7 @@ int op_fx_div(OraclePlan* p, const T* u, const T* v, const T* w, cudaStream_t st
   Launch L_(p, 0, st);
   if (p->z_fx)
     OB_CUDA((zfx<T, T>(ZFX_DIV, zline_x<T>(p), p->g, u, v, w, nullptr, 0.0, p->rho, p->rhoh,
-                       (C*)p->S1, (C*)p->S2, nullptr, st)));
+                       (C*)p->S1, (C*)p->S2, st)));
   else
     k_fx<T, FX_DIV><<<grid_x(p, p->zc_fx), kFftThreads, smem_fx(p, 3), st>>>(
         p->g, p->pxf, p->zc_fx, 3, u, v, w, nullptr, 0.0, p->rho, p->rhoh, p->theta0, p->kx,
@@ -2017,7 +2015,7 @@ int fwd_x(OraclePlan* p, const T* f, cudaStream_t st) {
   Launch L_(p, 0, st);
   if (p->z_fx)
     OB_CUDA((zfx<T, T>(ZFX_FIELDS, zline_x<T>(p), p->g, f, nullptr, nullptr, nullptr, 0.0, p->rho,
-                       p->rhoh, (C*)p->S1, nullptr, nullptr, st)));
+                       p->rhoh, (C*)p->S1, nullptr, st)));
   else
     k_fx<T, FX_FIELDS><<<grid_x(p, p->zc_fx), kFftThreads, smem_fx(p, 2), st>>>(
         p->g, p->pxf, p->zc_fx, 1, f, nullptr, nullptr, nullptr, 0.0, p->rho, p->rhoh, p->theta0,
@@ -2035,8 +2033,8 @@ int fwd_scalar(OraclePlan* p, const T* f, cudaStream_t st) {
   {
     Launch L_(p, 1, st);
     if (p->z_fy)
-      OB_CUDA((zfy<T, T>(ZFY_FIELDS, zline_y<T>(p), g, (C*)p->S1, nullptr, nullptr, 0.0, p->kx,
-                         p->ky, (C*)p->S3, nullptr, st)));
+      OB_CUDA((zfy<T, T>(ZFY_FIELDS, zline_y<T>(p), g, (C*)p->S1, nullptr, 0.0, p->kx, p->ky,
+                         (C*)p->S3, nullptr, st)));
     else
       k_fy<T, FY_FIELDS><<<grid_y(p, p->zc_fy), kFftThreads, smem_fy(p, 2, p->zc_fy), st>>>(
           g, p->pyf, p->zc_fy, 1, (C*)p->S1, nullptr, p->kx, p->ky, (const C*)p->twy, 1.0,
@@ -2708,8 +2706,8 @@ int vdiag_call(const OracleVortexDiag* d, int precision, const void* u, const vo
   return OB_OK;
 }
 
-// Uploads the level list after checking it is ascending inside [0, nz).
-// The band of an ascending level list; a list without gaps needs no upload.
+// The band of a level list that ascends inside [0, nz); only a list with gaps is
+// uploaded.
 int vdiag_levels(OracleVortexDiag* d, const int* lev, int nlev, VdBand* band, cudaStream_t st) {
   if (!lev || nlev < 1 || nlev > d->nz) return fail(OB_ERR_ARG, "vdiag: bad level list");
   for (int l = 0; l < nlev; ++l)

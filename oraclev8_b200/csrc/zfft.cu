@@ -69,8 +69,7 @@ using T = OB_ZREAL;
 template <class T, class TS, int RL>
 cudaError_t zfx_last(int mode, const ZLine<T>& l, const GridK& g, const TS* u, const TS* v,
                      const TS* w, const TS* bh, double sdt, const double* rho,
-                     const double* rhoh, cplx<T>* X0, cplx<T>* X1, cplx<T>* X2,
-                     cudaStream_t st);
+                     const double* rhoh, cplx<T>* X0, cplx<T>* X1, cudaStream_t st);
 template <class T, int RL>
 cudaError_t zix_last(int mode, const ZLine<T>& l, const GridK& g, const cplx<T>* S1,
                      const cplx<T>* S2, const T* u, const T* v, const T* w, const T* bh,
@@ -84,7 +83,6 @@ template <class T, int RL>
 cudaError_t zx_init() {
   OB_Z(attr(k_zfx<T, T, ZFX_DIV, RL>));
   OB_Z(attr(k_zfx<T, T, ZFX_STAGE, RL>));
-  OB_Z(attr(k_zfx<T, T, ZFX_SHARED, RL>));
   OB_Z(attr(k_zfx<T, T, ZFX_FIELDS, RL>));
   OB_Z(attr(k_zix<T, T, ZIX_CORRECT, RL>));
   OB_Z(attr(k_zix<T, T, ZIX_STAGE, RL>));
@@ -98,17 +96,15 @@ cudaError_t zx_init() {
 template <class T, class TS, int RL>
 cudaError_t zfx_last(int mode, const ZLine<T>& l, const GridK& g, const TS* u, const TS* v,
                      const TS* w, const TS* bh, double sdt, const double* rho,
-                     const double* rhoh, cplx<T>* X0, cplx<T>* X1, cplx<T>* X2,
-                     cudaStream_t st) {
+                     const double* rhoh, cplx<T>* X0, cplx<T>* X1, cudaStream_t st) {
   constexpr int C = zx_pairs<T>();
-  const int sets = mode == ZFX_FIELDS && !v ? 1 : mode == ZFX_SHARED ? 3 : 2;
+  const int sets = mode == ZFX_FIELDS && !v ? 1 : 2;
   const Shape s = shape<T>(l.plan, C, 1, g.ny, sets * div_up(g.nz, 2 * C), zx_threads<T>());
   const bool pairs = zpairs<TS>(g.nz, u, v);
 #define OB_ZFX(M)                                                                              \
   case M:                                                                                      \
     k_zfx<T, TS, M, RL><<<s.grid, s.threads, s.smem, st>>>(l.plan, g, s.rows, pairs, u, v, w, bh, \
-                                                           sdt, rho, rhoh, l.k, l.tw, X0, X1,  \
-                                                           X2);                                \
+                                                           sdt, rho, rhoh, l.k, l.tw, X0, X1); \
     break;
   if constexpr (sizeof(TS) != sizeof(T)) {
     switch (mode) { OB_ZFX(ZFX_DIV) default: return cudaErrorInvalidValue; }
@@ -116,7 +112,6 @@ cudaError_t zfx_last(int mode, const ZLine<T>& l, const GridK& g, const TS* u, c
     switch (mode) {
       OB_ZFX(ZFX_DIV)
       OB_ZFX(ZFX_STAGE)
-      OB_ZFX(ZFX_SHARED)
       OB_ZFX(ZFX_FIELDS)
       default: return cudaErrorInvalidValue;
     }
@@ -157,7 +152,7 @@ cudaError_t zix_last(int mode, const ZLine<T>& l, const GridK& g, const cplx<T>*
 #define OB_ZFX_INST(TS)                                                                       \
   template cudaError_t zfx_last<T, TS, OB_ZPART>(                                             \
       int, const ZLine<T>&, const GridK&, const TS*, const TS*, const TS*, const TS*, double, \
-      const double*, const double*, cplx<T>*, cplx<T>*, cplx<T>*, cudaStream_t);
+      const double*, const double*, cplx<T>*, cplx<T>*, cudaStream_t);
 OB_ZFX_INST(T)
 #if OB_ZWIDE
 OB_ZFX_INST(float)
@@ -178,10 +173,8 @@ cudaError_t zfft_init<T>() {
   constexpr int C = zy_cols<T>();
   OB_Z(attr(k_zfy<T>));
   OB_Z(attr(k_zfy2<T, T, ZFY_DIV, C>));
-  OB_Z(attr(k_zfy2<T, T, ZFY_SHARED, C>));
   OB_Z(attr(k_zfy2<T, T, ZFY_HELM, C>));
   OB_Z(attr(k_zfy2<T, T, ZFY_DIV, C / 2>));
-  OB_Z(attr(k_zfy2<T, T, ZFY_SHARED, C / 2>));
   OB_Z(attr(k_zfy2<T, T, ZFY_HELM, C / 2>));
   OB_Z(attr(k_ziy<T, true>));
   OB_Z(attr(k_ziy<T, false>));
@@ -206,9 +199,9 @@ cudaError_t zfft_init<T>() {
 template <class T, class TS>
 cudaError_t zfx(int mode, const ZLine<T>& l, const GridK& g, const TS* u, const TS* v,
                 const TS* w, const TS* bh, double sdt, const double* rho, const double* rhoh,
-                cplx<T>* X0, cplx<T>* X1, cplx<T>* X2, cudaStream_t st) {
+                cplx<T>* X0, cplx<T>* X1, cudaStream_t st) {
 #define OB_CALL(R) \
-  zfx_last<T, TS, R>(mode, l, g, u, v, w, bh, sdt, rho, rhoh, X0, X1, X2, st)
+  zfx_last<T, TS, R>(mode, l, g, u, v, w, bh, sdt, rho, rhoh, X0, X1, st)
   OB_ZLASTS(OB_CALL)
 #undef OB_CALL
 }
@@ -226,35 +219,33 @@ cudaError_t zix(int mode, const ZLine<T>& l, const GridK& g, const cplx<T>* S1,
 // two lines per column: full columns where two CTAs per SM hold them
 template <class T, class TO, int MODE>
 cudaError_t zfy2(const ZLine<T>& l, const GridK& g, const cplx<T>* X0, const cplx<T>* X1,
-                 const cplx<T>* X2, double sc, const double* kxd, const double* kyd,
+                 double sc, const double* kxd, const double* kyd,
                  cplx<TO>* out0, cplx<T>* out1, cudaStream_t st) {
   constexpr int C = zy_cols<T>();
   if (2ull * l.plan.NP * C * 2 * sizeof(T) <= kZSmemMax / 2) {
     const Shape s = shape<T>(l.plan, C, 2, g.nxh, div_up(g.nz, C), kZThreads);
     k_zfy2<T, TO, MODE, C><<<s.grid, s.threads, s.smem, st>>>(
-        l.plan, g, s.rows, X0, X1, X2, sc, l.k, kxd, kyd, l.tw, out0, out1);
+        l.plan, g, s.rows, X0, X1, sc, l.k, kxd, kyd, l.tw, out0, out1);
   } else {
     const Shape s = shape<T>(l.plan, C / 2, 2, g.nxh, div_up(g.nz, C / 2), kZThreads);
     k_zfy2<T, TO, MODE, C / 2><<<s.grid, s.threads, s.smem, st>>>(
-        l.plan, g, s.rows, X0, X1, X2, sc, l.k, kxd, kyd, l.tw, out0, out1);
+        l.plan, g, s.rows, X0, X1, sc, l.k, kxd, kyd, l.tw, out0, out1);
   }
   return cudaGetLastError();
 }
 
 template <class T, class TO>
 cudaError_t zfy(int mode, const ZLine<T>& l, const GridK& g, const cplx<T>* X0,
-                const cplx<T>* X1, const cplx<T>* X2, double sc, const double* kxd,
+                const cplx<T>* X1, double sc, const double* kxd,
                 const double* kyd, cplx<TO>* out0, cplx<T>* out1, cudaStream_t st) {
   if constexpr (sizeof(TO) != sizeof(T)) {
     if (mode != ZFY_RESID) return cudaErrorInvalidValue;
-    return zfy2<T, TO, ZFY_RESID>(l, g, X0, X1, X2, sc, kxd, kyd, out0, out1, st);
+    return zfy2<T, TO, ZFY_RESID>(l, g, X0, X1, sc, kxd, kyd, out0, out1, st);
   } else {
     if (mode == ZFY_DIV)
-      return zfy2<T, TO, ZFY_DIV>(l, g, X0, X1, X2, sc, kxd, kyd, out0, out1, st);
-    if (mode == ZFY_SHARED)
-      return zfy2<T, TO, ZFY_SHARED>(l, g, X0, X1, X2, sc, kxd, kyd, out0, out1, st);
+      return zfy2<T, TO, ZFY_DIV>(l, g, X0, X1, sc, kxd, kyd, out0, out1, st);
     if (mode == ZFY_HELM)
-      return zfy2<T, TO, ZFY_HELM>(l, g, X0, X1, X2, sc, kxd, kyd, out0, out1, st);
+      return zfy2<T, TO, ZFY_HELM>(l, g, X0, X1, sc, kxd, kyd, out0, out1, st);
     if (mode != ZFY_FIELDS) return cudaErrorInvalidValue;
     constexpr int C = zy_cols<T>();
     const Shape s = shape<T>(l.plan, C, 1, g.nxh, div_up(g.nz, C), kZThreads);
@@ -318,10 +309,10 @@ cudaError_t zplane_inv(const GridK& g, const ThomasK& t, double* inv, cudaStream
 #define OB_ZFX_INST(TS)                                                                      \
   template cudaError_t zfx<T, TS>(int, const ZLine<T>&, const GridK&, const TS*, const TS*,  \
                                   const TS*, const TS*, double, const double*, const double*, \
-                                  cplx<T>*, cplx<T>*, cplx<T>*, cudaStream_t);
+                                  cplx<T>*, cplx<T>*, cudaStream_t);
 #define OB_ZFY_INST(TO)                                                                      \
   template cudaError_t zfy<T, TO>(int, const ZLine<T>&, const GridK&, const cplx<T>*,        \
-                                  const cplx<T>*, const cplx<T>*, double, const double*,     \
+                                  const cplx<T>*, double, const double*,                     \
                                   const double*, cplx<TO>*, cplx<T>*, cudaStream_t);
 OB_ZFX_INST(T)
 OB_ZFY_INST(T)

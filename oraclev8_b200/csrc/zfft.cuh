@@ -529,17 +529,15 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
     const __grid_constant__ ZPlan p, GridK g, int RY, bool pairs, const TS* __restrict__ u,
     const TS* __restrict__ v, const TS* __restrict__ w, const TS* __restrict__ bh, double sdt,
     const double* __restrict__ rho, const double* __restrict__ rhoh, const T* __restrict__ kx,
-    const cplx<T>* __restrict__ tw, cplx<T>* __restrict__ X0, cplx<T>* __restrict__ X1,
-    cplx<T>* __restrict__ X2) {
+    const cplx<T>* __restrict__ tw, cplx<T>* __restrict__ X0, cplx<T>* __restrict__ X1) {
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   constexpr int C = zx_pairs<T>();
   constexpr int LC = zlog2(C);
   cplx<T>* b0 = reinterpret_cast<cplx<T>*>(smem_dyn);
   const int ny = g.ny, nz = g.nz;
   const int y0 = blockIdx.y * RY;
-  // line sets, a block each: rho u with D w, rho v, the shared form's D b_half
-  constexpr int SETS = MODE == ZFX_SHARED ? 3 : 2;
-  const int sets = MODE == ZFX_FIELDS && !v ? 1 : SETS;
+  // line sets, a block each: rho u with D w, and rho v
+  const int sets = MODE == ZFX_FIELDS && !v ? 1 : 2;
   const int chunk = blockIdx.x / sets, set = blockIdx.x - chunk * sets;
   const int z = (chunk * C + (threadIdx.x & (C - 1))) * 2;  // the thread's first level
   const bool on = z < nz, two = z + 1 < nz, vec = pairs;
@@ -571,7 +569,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
     };
   };
   // vertical flux divergence of w (STAGE: of w + sdt b_half)
-  auto flux = [&](const TS* f, const TS* b) {
+  auto flux = [&]() {
     return [=](auto rc, int row, int c, int n, int step, cplx<T>* r) {
       constexpr int R = decltype(rc)::value;
       if (!on || row >= rows) return;
@@ -579,7 +577,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
       T w0[R], w1[R], w2[R];
 #pragma unroll
       for (int j = 0; j < R; ++j) {
-        const TS* q = f + o + j * step * ws;
+        const TS* q = w + o + j * step * ws;
         w0[j] = (T)q[0];
         w1[j] = (T)q[1];
         w2[j] = two ? (T)q[2] : (T)0;
@@ -587,7 +585,7 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
 #pragma unroll
       for (int j = 0; j < R; ++j) {
         if (MODE == ZFX_STAGE) {
-          const TS* q = b + o + j * step * ws;
+          const TS* q = bh + o + j * step * ws;
           const zval<T> s0 = zstage(w0[j], sd, (T)q[0]), s1 = zstage(w1[j], sd, (T)q[1]);
           const zval<T> s2 = zstage(w2[j], sd, two ? (T)q[2] : (T)0);
           r[j] = mk<T>(wdiff(f1, s1, f0, s0), two ? wdiff(f2, s2, f1, s1) : (T)0);
@@ -605,9 +603,9 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zfx(
     const bool sum = run == 1;
     if (sum && set) return;
     const bool grad = MODE != ZFX_FIELDS && set == 0 && !sum;  // times i kx'
-    cplx<T>* out = set == 0 ? X0 : set == 1 ? X1 : X2;
+    cplx<T>* out = set == 0 ? X0 : X1;
     if (run) __syncthreads();
-    if (MODE != ZFX_FIELDS && (sum || set == 2)) z_first_fwd<T, C>(p, b0, RY, flux(sum ? w : bh, bh));
+    if (MODE != ZFX_FIELDS && sum) z_first_fwd<T, C>(p, b0, RY, flux());
     else z_first_fwd<T, C>(p, b0, RY, field(set ? v : u, MODE != ZFX_FIELDS));
     __syncthreads();
 #pragma unroll 1
@@ -901,12 +899,10 @@ __global__ void __launch_bounds__(zx_threads<T>(), zx_blocks<T>()) k_zix(
 // ---- y lines ---------------------------------------------------------------------
 // One level of one kx per column; rows of a CTA are consecutive kx.
 
-// rows of a spectrum at one level (times s added from another) into a line's
-// first forward pass
+// rows of a spectrum at one level into a line's first forward pass
 template <class T, int C>
 __device__ __forceinline__ void zy_first(const ZPlan& p, const GridK& g, cplx<T>* buf, int RY,
-                                         int rows, int k0, int z, const cplx<T>* src,
-                                         const cplx<T>* add_, T sc) {
+                                         int rows, int k0, int z, const cplx<T>* src) {
   const bool on = z < g.nz;
   z_first_fwd<T, C>(p, buf, RY, [&](auto rc, int row, int c, int n, int step, cplx<T>* v) {
     constexpr int R = decltype(rc)::value;
@@ -914,13 +910,6 @@ __device__ __forceinline__ void zy_first(const ZPlan& p, const GridK& g, cplx<T>
     const int o = ((k0 + row) * g.ny + n) * g.nz + z;
 #pragma unroll
     for (int j = 0; j < R; ++j) v[j] = src[o + j * step * g.nz];
-    if (add_) {
-      cplx<T> a[R];
-#pragma unroll
-      for (int j = 0; j < R; ++j) a[j] = add_[o + j * step * g.nz];
-#pragma unroll
-      for (int j = 0; j < R; ++j) v[j] = mk<T>(v[j].x + sc * a[j].x, v[j].y + sc * a[j].y);
-    }
   });
 }
 
@@ -956,7 +945,7 @@ __global__ void __launch_bounds__(kZThreads, sizeof(T) == 4 ? 3 : 2) k_zfy(
   const int z = blockIdx.x * C + (threadIdx.x & (C - 1));
   const bool on = z < nz;
   const int rows = min(RY, g.nxh - k0);
-  zy_first<T, C>(p, g, b0, RY, rows, k0, z, X0, nullptr, (T)0);
+  zy_first<T, C>(p, g, b0, RY, rows, k0, z, X0);
   __syncthreads();
 #pragma unroll 1
   for (int i = 1; i + 1 < p.np; ++i) {
@@ -982,14 +971,12 @@ __global__ void __launch_bounds__(kZThreads, sizeof(T) == 4 ? 3 : 2) k_zfy(
   });
 }
 
-// Forward y of two fields, both lines in shared memory: ZFY_DIV, ZFY_SHARED,
-// ZFY_RESID (the sum rounded to TO once) and ZFY_HELM (multipliers that mix the
+// Forward y of two fields, both lines in shared memory: ZFY_DIV, ZFY_RESID (the sum rounded to TO once) and ZFY_HELM (multipliers that mix the
 // two, then both lines back).
 template <class T, class TO, int MODE, int C>
 __global__ void __launch_bounds__(kZThreads, sizeof(T) == 4 ? 3 : 2) k_zfy2(
     const __grid_constant__ ZPlan p, GridK g, int RY, const cplx<T>* X0, const cplx<T>* X1,
-    const cplx<T>* __restrict__ X2, double s_, const T* __restrict__ ky,
-    const double* __restrict__ kxd,
+    double s_, const T* __restrict__ ky, const double* __restrict__ kxd,
     const double* __restrict__ kyd, const cplx<T>* __restrict__ tw, cplx<TO>* out0,
     cplx<T>* out1) {
   extern __shared__ __align__(16) unsigned char smem_dyn[];
@@ -1003,8 +990,7 @@ __global__ void __launch_bounds__(kZThreads, sizeof(T) == 4 ? 3 : 2) k_zfy2(
   const int rows = min(RY, g.nxh - k0);
 #pragma unroll
   for (int f = 0; f < 2; ++f)
-    zy_first<T, C>(p, g, f ? b1 : b0, RY, rows, k0, z, f ? X1 : X0,
-                   MODE == ZFY_SHARED && !f ? X2 : nullptr, (T)s_);
+    zy_first<T, C>(p, g, f ? b1 : b0, RY, rows, k0, z, f ? X1 : X0);
   __syncthreads();
 #pragma unroll 1
   for (int i = 1; i + 1 < p.np; ++i) {

@@ -21,8 +21,8 @@ struct ZPlan {
 };
 
 // The plan of an even line of N points with elements of `elem` bytes (4 or 8);
-// false where N has no factorisation in the kernels' radices or two buffers of
-// one line exceed shared memory.
+// false where N has no factorisation in the kernels' radices or a line of every
+// column exceeds shared memory.
 bool zplan_make(int N, int elem, ZPlan* out);
 
 // The index into W_N^t of every entry of the line's pass twiddles (N entries).
@@ -49,8 +49,7 @@ struct ZLine {
 // forward x modes
 #define ZFX_DIV 0     // X0 = i kx' F(rho u) + F(D w), X1 = F(rho v)
 #define ZFX_STAGE 1   // the same of w + sdt b_half
-#define ZFX_SHARED 2  // ZFX_DIV and X2 = F(D b_half)
-#define ZFX_FIELDS 3  // X0 = F(u), X1 = F(v) (v null: X0 alone)
+#define ZFX_FIELDS 2  // X0 = F(u), X1 = F(v) (v null: X0 alone)
 // inverse x modes
 #define ZIX_CORRECT 0  // u, v, w -= grad phi; phi stored unless null
 #define ZIX_STAGE 1    // out = (u, v, w + sdt b_half) - grad phi
@@ -59,10 +58,9 @@ struct ZLine {
 #define ZIX_GRAD 4     // uo, vo, wo = the gradient (wo on nz + 1 levels, 0 at the ends)
 // forward y modes
 #define ZFY_DIV 0     // out0 = F(X0) + i ky' F(X1)
-#define ZFY_SHARED 1  // out0 = F(X0 + s X2) + i ky' F(X1): a fast stage
-#define ZFY_RESID 2   // ZFY_DIV, zero on the Nyquist rows, rounded to TO
-#define ZFY_FIELDS 3  // out0 = F(X0)
-#define ZFY_HELM 4    // forward, the damper's multipliers (times s), and back
+#define ZFY_RESID 1   // ZFY_DIV, zero on the Nyquist rows, rounded to TO
+#define ZFY_FIELDS 2  // out0 = F(X0)
+#define ZFY_HELM 3    // forward, the damper's multipliers (times s), and back
 
 // Raises the kernels' shared-memory limits on the current device.
 template <class T>
@@ -71,14 +69,14 @@ cudaError_t zfft_init();
 template <class T, class TS>
 cudaError_t zfx(int mode, const ZLine<T>& l, const GridK& g, const TS* u, const TS* v,
                 const TS* w, const TS* bh, double sdt, const double* rho, const double* rhoh,
-                cplx<T>* X0, cplx<T>* X1, cplx<T>* X2, cudaStream_t st);
+                cplx<T>* X0, cplx<T>* X1, cudaStream_t st);
 template <class T>
 cudaError_t zix(int mode, const ZLine<T>& l, const GridK& g, const cplx<T>* S1,
                 const cplx<T>* S2, const T* u, const T* v, const T* w, const T* bh, double sdt,
                 T* uo, T* vo, T* wo, T* phio, cudaStream_t st);
 template <class T, class TO>
 cudaError_t zfy(int mode, const ZLine<T>& l, const GridK& g, const cplx<T>* X0,
-                const cplx<T>* X1, const cplx<T>* X2, double s, const double* kxd,
+                const cplx<T>* X1, double s, const double* kxd,
                 const double* kyd, cplx<TO>* out0, cplx<T>* out1, cudaStream_t st);
 template <class T>
 cudaError_t ziy(bool grad, const ZLine<T>& l, const GridK& g, const cplx<T>* in, double scale,
