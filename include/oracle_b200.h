@@ -129,7 +129,10 @@ extern "C" {
                              * takes effect with the 1024-point y pencils (zc4_fy) */
 /* The level-paired line transforms (any nx, ny whose halves have no factor
  * above 5), 0 or 1 per class; a class whose entry is 1 runs them whatever its
- * other entries are.  _FXD / _FYD: the FP64 residual transforms. */
+ * other entries are.  _FXD / _FYD: the FP64 residual transforms.  Setting the
+ * first n choices turns off the level-paired entries from n on whose class has
+ * another entry below n: an array that ends before them chooses among the
+ * forms that it names. */
 #define OB_VAR_Z_FX 23
 #define OB_VAR_Z_FXS 24
 #define OB_VAR_Z_IX 25

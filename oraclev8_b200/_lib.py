@@ -48,6 +48,18 @@ VARIANTS = ("zc2_fx", "zc2_fxs", "zc2_ix", "zc2_fy", "zc2_iy", "zc3_fx", "zc3_fx
             "zc4_iy", "slow_xw", "thomas_fast", "rzc2_fx", "rzc2_fy", "zc4_fyd", "zc4_fxsh", "z_fx",
             "z_fxs", "z_ix", "z_fy", "z_iy", "z_fxd", "z_fyd",
             "z_yz")
+# the older forms that each level-paired form runs instead of; the plane form's
+# are those of both y transforms and of the solve between them
+OLDER_FORMS = {
+    "z_fx": ("zc4_fx", "zc3_fx", "zc2_fx"),
+    "z_fxs": ("zc4_fxs", "zc3_fxs", "zc2_fxs"),
+    "z_ix": ("zc4_ix", "zc3_ix", "zc2_ix"),
+    "z_fy": ("zc4_fy", "zc3_fy", "zc2_fy"),
+    "z_iy": ("zc4_iy", "zc3_fy", "zc2_iy"),
+    "z_fxd": ("zc4_fxd", "zc3_fxd", "rzc2_fx"),
+    "z_fyd": ("zc4_fyd", "zc3_fyd", "rzc2_fy"),
+    "z_yz": ("zc4_fy", "zc3_fy", "zc2_fy", "zc4_iy", "zc2_iy", "thomas_fast"),
+}
 OB_TUNE_FORCE = 1
 ABI_VERSION = 3  # OB_ABI_VERSION of the header these tables follow
 PROF_CLASSES = ("fx", "fy", "thomas", "iy", "ix", "slow", "diag", "other", "refine",

@@ -205,8 +205,13 @@ class Plan:
 
     def set_variants(self, **kw) -> None:
         """Change some choices (``plan.set_variants(zc4_ix=8)``); every value is
-        checked against the forms the plan's grid and precision allow."""
+        checked against the forms the plan's grid and precision allow.  Naming
+        one of a class's older forms chooses among those: the level-paired
+        form, which would run instead of them, goes off unless it is named too."""
         cur = self.variants()
+        for z, older in L.OLDER_FORMS.items():
+            if any(k in kw for k in older):
+                cur[z] = 0
         for k, v in kw.items():
             if k not in cur:
                 raise ValueError(f"unknown kernel variant {k!r}")

@@ -3536,6 +3536,24 @@ int oracle_b200_plan_set_variants(OraclePlan* p, const int* in, int n) {
   for (int i = 0; i < n; ++i)
     if (!var_allowed(p, i, in[i]))
       return fail(OB_ERR_ARG, "plan_set_variants: variant %d cannot be %d on this plan", i, in[i]);
+  // a level-paired form beyond the array would run instead of those it chooses
+  static const struct {
+    int z;
+    std::vector<int> older;
+  } kPaired[] = {
+      {OB_VAR_Z_FX, {OB_VAR_ZC4_FX, OB_VAR_ZC3_FX, OB_VAR_ZC2_FX}},
+      {OB_VAR_Z_FXS, {OB_VAR_ZC4_FXS, OB_VAR_ZC3_FXS, OB_VAR_ZC2_FXS}},
+      {OB_VAR_Z_IX, {OB_VAR_ZC4_IX, OB_VAR_ZC3_IX, OB_VAR_ZC2_IX}},
+      {OB_VAR_Z_FY, {OB_VAR_ZC4_FY, OB_VAR_ZC3_FY, OB_VAR_ZC2_FY}},
+      {OB_VAR_Z_IY, {OB_VAR_ZC4_IY, OB_VAR_ZC3_FY, OB_VAR_ZC2_IY}},
+      {OB_VAR_Z_FXD, {OB_VAR_ZC4_FXD, OB_VAR_ZC3_FXD, OB_VAR_RZC2_FX}},
+      {OB_VAR_Z_FYD, {OB_VAR_ZC4_FYD, OB_VAR_ZC3_FYD, OB_VAR_RZC2_FY}},
+      {OB_VAR_Z_YZ,
+       {OB_VAR_ZC4_FY, OB_VAR_ZC3_FY, OB_VAR_ZC2_FY, OB_VAR_ZC4_IY, OB_VAR_ZC2_IY,
+        OB_VAR_THOMAS_FAST}}};
+  for (const auto& c : kPaired)
+    for (int o : c.older)
+      if (o < n && c.z >= n) *var_field(p, c.z) = 0;
   for (int i = 0; i < n; ++i)
     if (int* f = var_field(p, i)) *f = in[i];
   return OB_OK;
