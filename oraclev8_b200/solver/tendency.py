@@ -282,9 +282,9 @@ class AnelasticProjection(ProjectionComponent):
         self._solve_count += 1
         de = max(1, int(os.environ.get("ORACLE_POISSON_DIAG_EVERY", "60")))
         log = de == 1 or self._solve_count % de == 1
-        # straight from the state's fields into new ones; a field that the kernels' loads
-        # cannot take as it lies (strides, a view off 16 bytes) goes through a copy.  The three
-        # copies took 60 of 520 us at 384 x 384 x 48 in FP64
+        # straight from the state's fields into new ones; a field with strides goes through a
+        # copy, and so does a view off 16 bytes, which would lose the kernels' paired loads.
+        # The three copies took 60 of 520 us at 384 x 384 x 48 in FP64
         ins = [a if a.is_contiguous() and a.data_ptr() % 16 == 0 else a.clone()
                for a in (state.u, state.v, state.w)]
         u, v, w = (torch.empty_like(a) for a in ins)
